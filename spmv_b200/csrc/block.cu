@@ -2,43 +2,264 @@
 // reference; builds on Matrix::operator* and spmv::cg, cg.cpp:11-83).
 //
 // Vectors of k right-hand sides are stored row-major (n x k, leading
-// dimension k), so the k values of one row are contiguous.  The SpMM gives a
-// row a group of K lanes (K = k rounded up to a power of two, at most 32):
-// every lane reads the row's column indices and values (the same addresses,
-// one broadcast transaction) and lane l accumulates right-hand side l from a
-// contiguous run of X.  A is read once for all k right-hand sides.
+// dimension k), so the k values of one row are contiguous.  A row is computed
+// by a group of KL lanes, each with a run of right-hand sides (Run below:
+// 16-byte accesses of X and Y where k and the vectors' alignment allow); every
+// lane of the group reads the row's columns and values (one broadcast
+// transaction).  A is read once for all k right-hand sides.
+//
+// What bounds the product: X is gathered from L2, 8 k bytes per entry, behind
+// a chain of dependent loads (row pointer, column, X).  So each lane keeps
+// SPMM_BATCH entries in flight and issues every batch whole (a tail of single
+// entries costs one chain each), the next row's pointers are loaded a row
+// ahead, and a CTA takes chunks of neighbouring rows (RowChunks).  Rows longer
+// than LONG_ROW entries are left to the whole CTA.  Against one right-hand
+// side per lane, batches of four and a tail (FP64, 7-point 96^3, 4 ranks):
+// k = 2 24.7 -> 20.2 us, k = 8 69.8 -> 59.3, k = 16 133 -> 104 (3.0 TB/s of
+// compulsory traffic), k = 32 250 -> 189; with rows of up to 12,500 entries
+// (100,003 power-law rows, k = 8) 1.38 ms -> 70 us.
 //
 // Block CG runs k independent CG recurrences that share each product: the
 // SpMM's epilogue forms the k dot products p_l . (A p)_l, and every column has
 // its own alpha, beta, convergence test (cg.cpp:78) and breakdown flag; a
 // converged column stops changing.  The loop ends when every column has
-// converged or broken down, or after max_its iterations, as one CUDA graph
-// with a device-side while loop (same structure as cg.cu).
+// converged or broken down, or after max_its iterations.  A solve is one
+// cooperative launch of persistent CTAs (one per SM: grid sums cost more with
+// every CTA that takes part; k = 2 on 250k rows, 24 us per iteration with three
+// CTAs of 256 threads per SM, 19 with one of 1024) with two grid sums of k
+// values and one grid barrier per iteration, the same form as the fused single
+// solve (cg.cu).  Its workspace is kept with the matrix.  Per iteration on
+// 64 x 64 x 61, 4 ranks: k = 1 17.8 us, k = 8 39, k = 32 160; as a CUDA graph
+// of three kernels whose column sums one thread added over the grid, 120-160,
+// 217 and 425.
 #include <algorithm>
 #include <cmath>
 
 #include "internal.h"
 #include "spmv_kernel.cuh"
 
+struct BlockWorkspace {
+  int64_t n = 0;
+  // b, x, r, p, y (n x k, for the largest k solved so far), per-CTA partials,
+  // state and the grid barrier's counter.
+  spmvb::DevBuf b, x, r, p, y, partials, state;
+};
+
 namespace spmvb {
 
 namespace {
 
-constexpr int BBS = 256;
+constexpr int BBS = 256;       // threads per CTA
+constexpr int BCPS = 4;            // CTAs per SM the block product is compiled to fit
+constexpr int CBS = 1024;          // threads per CTA of block CG, one CTA per SM
 constexpr int MAXK = 32;
+constexpr int SPMM_BATCH = 8;      // entries in flight per lane
+constexpr int LONG_ROW = 512;      // entries above which a row is the whole CTA's
+// Values of X per chunk of rows: the product's chunks keep their X rows and
+// their neighbours' in L1; the solver's are one per CTA up to this size (its
+// vectors then stay in L2 between the phases).
+constexpr int SPMM_CHUNK = 4096, BCG_CHUNK = 24576;
 
-// Rows of one launch: group of K lanes per row, lane = right-hand side.
-template <typename T, int K, class F>
-__device__ __forceinline__ void spmm_rows(const SpmvArgs& a, int k, F&& f) {
+// Right-hand sides per lane.  V consecutive ones, the vectors aligned to V
+// values (SPLIT false); or two, loaded one by one, the second missing from
+// the last lane of an odd k (SPLIT).
+template <int V_, bool SPLIT_>
+struct Run {
+  static constexpr int V = V_;
+  static constexpr bool SPLIT = SPLIT_;
+  int c0;    // first right-hand side
+  int next;  // SPLIT: offset of the second (0 when there is none)
+  bool on;
+  __device__ __forceinline__ Run(int member, int k)
+      : c0(member * V), next(member * V + 1 < k ? 1 : 0), on(member * V < k) {}
+};
+
+template <typename T, class R>
+__device__ __forceinline__ void ld_run(const R& r, const T* p, T (&o)[R::V]) {
+  if constexpr (R::V == 1) {
+    o[0] = *p;
+  } else if constexpr (R::SPLIT) {
+    o[0] = p[0];
+    o[1] = p[r.next];
+  } else if constexpr (sizeof(T) * R::V == 16) {
+    const typename VecT<T>::V t = *reinterpret_cast<const typename VecT<T>::V*>(p);
+#pragma unroll
+    for (int i = 0; i < R::V; ++i) o[i] = comp(t, i);
+  } else {
+    const float2 t = *reinterpret_cast<const float2*>(p);
+    o[0] = t.x;
+    o[1] = t.y;
+  }
+}
+template <typename T, class R>
+__device__ __forceinline__ void st_run(const R& r, T* p, const T (&v)[R::V]) {
+  if constexpr (R::V == 1) {
+    *p = v[0];
+  } else if constexpr (R::SPLIT) {
+    p[0] = v[0];
+    if (r.next) p[1] = v[1];
+  } else if constexpr (sizeof(T) == 8) {
+    *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+  } else if constexpr (R::V == 4) {
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  } else {
+    *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+  }
+}
+
+// Rows are dealt to the CTAs in chunks of consecutive rows (global numbering):
+// chunk q is [q rows, (q + 1) rows).  A chunk's neighbouring rows share X rows
+// in the CTA's L1, and chunks in flight are consecutive, so the X rows that
+// rows further apart share (the next plane of a grid) are read from DRAM
+// once.
+struct RowChunks {
+  int64_t rows, total;  // rows per chunk, rows in all
+  int count;
+  __host__ __device__ int64_t begin(int64_t q) const { return q * rows; }
+  __host__ __device__ int64_t end(int64_t q) const {
+    return (q + 1) * rows < total ? (q + 1) * rows : total;
+  }
+};
+
+// acc += the row's entries below e from j on, in batches of SPMM_BATCH
+// consecutive entries at j, j + step, ...  Every batch is issued whole: past
+// the end it repeats the last entry and the sum skips it.  (X may be written
+// between the calls of one launch, so it is read with ordinary loads.)
+template <typename T, class R>
+__device__ __forceinline__ void spmm_entries(const R& r, const int32_t* cols, const T* vals,
+                                             const T* xc, int k, int j, int e, int step,
+                                             T (&acc)[R::V]) {
+  constexpr int BU = SPMM_BATCH;
+  for (; j < e; j += step) {
+    int c[BU];
+    T v[BU], xv[BU][R::V];
+#pragma unroll
+    for (int u = 0; u < BU; ++u) c[u] = __ldg(cols + min(j + u, e - 1));
+#pragma unroll
+    for (int u = 0; u < BU; ++u) ld_run<T>(r, xc + int64_t(c[u]) * k, xv[u]);
+#pragma unroll
+    for (int u = 0; u < BU; ++u) v[u] = __ldg(vals + min(j + u, e - 1));
+#pragma unroll
+    for (int u = 0; u < BU; ++u)
+      if (j + u < e)
+#pragma unroll
+        for (int i = 0; i < R::V; ++i) acc[i] += v[u] * xv[u][i];
+  }
+}
+
+// Rows [g0, g1) (global numbering) of Y = A X, by the whole CTA, KL lanes per
+// row: f(P, row, run, sums) once per row and lane that has right-hand sides.
+template <typename T, int NT, int KL, class R, class F>
+__device__ __forceinline__ void spmm_rows(const SpmvArgs& a, int k, int64_t g0, int64_t g1,
+                                          F&& f) {
+  constexpr int V = R::V;
+  __shared__ T group_sums[NT * V];
+  __shared__ unsigned int long_mask[NT / 32];
+  const int tid = int(threadIdx.x), grp = tid / KL;
+  const R run(tid % KL, k);
+  int64_t row0 = 0;
+  for (int p = 0; p < a.nparts; ++p) {
+    const PartArg& P = a.part[p];
+    const int64_t first = row0;
+    row0 += P.nrows;
+    const int lo = int(max(g0, first) - first), hi = int(min(g1, row0) - first);
+    if (g0 >= row0 || g1 <= first || lo >= hi) continue;
+    const T* xc = static_cast<const T*>(P.x) + (run.on ? run.c0 : 0);
+    const T* vals = static_cast<const T*>(P.vals);
+    int row = lo + grp;
+    int s = 0, e = 0, any_long = 0;
+    if (row < hi) {
+      s = __ldg(P.rowptr + row);
+      e = __ldg(P.rowptr + row + 1);
+    }
+    while (row < hi) {
+      const int next = row + NT / KL;
+      int sn = 0, en = 0;
+      if (next < hi) {
+        sn = __ldg(P.rowptr + next);
+        en = __ldg(P.rowptr + next + 1);
+      }
+      if (e - s > LONG_ROW) {
+        any_long = 1;
+      } else {
+        T acc[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) acc[i] = T(0);
+        spmm_entries<T>(run, P.cols, vals, xc, k, s, e, SPMM_BATCH, acc);
+        if (run.on) f(P, row, run, acc);
+      }
+      row = next;
+      s = sn;
+      e = en;
+    }
+    if (!__syncthreads_or(any_long)) continue;
+    // Long rows, in row order: every group takes batches in
+    // turn; the groups' sums are added in group order.
+    for (int r0 = lo; r0 < hi; r0 += NT) {
+      const int mine = r0 + tid;
+      const bool is_long =
+          mine < hi && __ldg(P.rowptr + mine + 1) - __ldg(P.rowptr + mine) > LONG_ROW;
+      const unsigned int m = __ballot_sync(0xffffffffu, is_long);
+      if ((tid & 31) == 0) long_mask[tid >> 5] = m;
+      __syncthreads();
+      for (int w = 0; w < NT / 32; ++w)
+        for (unsigned int left = long_mask[w]; left != 0; left &= left - 1) {
+          const int lrow = r0 + 32 * w + __ffs(left) - 1;
+          const int ls = __ldg(P.rowptr + lrow), le = __ldg(P.rowptr + lrow + 1);
+          T acc[V];
+#pragma unroll
+          for (int i = 0; i < V; ++i) acc[i] = T(0);
+          spmm_entries<T>(run, P.cols, vals, xc, k, ls + grp * SPMM_BATCH, le,
+                          SPMM_BATCH * (NT / KL), acc);
+#pragma unroll
+          for (int i = 0; i < V; ++i) group_sums[tid * V + i] = acc[i];
+          __syncthreads();
+          if (grp == 0 && run.on) {
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+              T t = T(0);
+              for (int g = 0; g < NT / KL; ++g) t += group_sums[g * KL * V + run.c0 + i];
+              acc[i] = t;
+            }
+            f(P, lrow, run, acc);
+          }
+          __syncthreads();
+        }
+      __syncthreads();
+    }
+  }
+}
+
+template <typename T, int KL, class R>
+__global__ void __launch_bounds__(BBS, BCPS)
+    spmm_kernel(const __grid_constant__ SpmvArgs a, const RowChunks ch, int k) {
+  spmm_rows<T, BBS, KL, R>(a, k, ch.begin(blockIdx.x), ch.end(blockIdx.x),
+                           [&](const PartArg& P, int row, const R& run, const T(&acc)[R::V]) {
+                             st_run<T>(run, static_cast<T*>(P.y) + int64_t(row) * k + run.c0,
+                                       acc);
+                           });
+}
+
+// One right-hand side per lane, KL lanes per row, CTAs striding over tiles of
+// BBS / KL rows; batches of four entries and a tail of single ones, in 32
+// registers (every warp slot of the SM taken).  For an odd number of
+// right-hand sides (or vectors off a 16-byte boundary) on rows of several
+// batches, where twice the warps are worth more than two right-hand sides
+// per lane loaded one by one (FP64, 60^3 rows: k = 7, 27-point 51 us against
+// 58, mesh 34 against 43; k = 31, 148 against 172 and 91 against 102; rows of
+// 7 entries, 96^3: k = 7, 70 against 66, k = 31, 255 against 219).
+template <typename T, int KL>
+__global__ void __launch_bounds__(BBS)
+    spmm_walk_kernel(const __grid_constant__ SpmvArgs a, int k) {
   const int p = find_part(a, blockIdx.x);
   const PartArg& P = a.part[p];
   const int32_t* __restrict__ cols = P.cols;
   const T* __restrict__ vals = static_cast<const T*>(P.vals);
   const T* __restrict__ x = static_cast<const T*>(P.x);
-  const int group = int(threadIdx.x) / K, lane = int(threadIdx.x) % K;
+  const int group = int(threadIdx.x) / KL, lane = int(threadIdx.x) % KL;
   const bool on = lane < k;
   for (int tile = int(blockIdx.x) - P.block_begin; tile < P.ntiles; tile += P.nblocks) {
-    const int row = tile * (BBS / K) + group;
+    const int row = tile * (BBS / KL) + group;
     if (row >= P.nrows) continue;
     const int s = __ldg(P.rowptr + row), e = __ldg(P.rowptr + row + 1);
     T acc = T(0);
@@ -61,27 +282,18 @@ __device__ __forceinline__ void spmm_rows(const SpmvArgs& a, int k, F&& f) {
       const T v = __ldg(vals + j);
       if (on) acc += v * __ldg(x + int64_t(c) * k + lane);
     }
-    if (on) f(P, row, lane, acc);
+    if (on) static_cast<T*>(P.y)[int64_t(row) * k + lane] = acc;
   }
 }
 
-template <typename T, int K>
-__global__ void __launch_bounds__(BBS)
-    spmm_kernel(const __grid_constant__ SpmvArgs a, int k) {
-  spmm_rows<T, K>(a, k, [&](const PartArg& P, int row, int lane, T acc) {
-    static_cast<T*>(P.y)[int64_t(row) * k + lane] = acc;
-  });
-}
-
 // ---------------------------------------------------------------------------
-// Block CG state and kernels
+// Block CG
 // ---------------------------------------------------------------------------
 struct BcgState {
-  double rr0[MAXK], rr[MAXK], pap[MAXK], alpha[MAXK], beta[MAXK];
-  int active[MAXK], status[MAXK], its[MAXK];
-  int k, kmax, nrhs, pad;
-  double rtol2;
-  unsigned int t0, t1, t2, pad2;
+  double rr0[MAXK], rr[MAXK];
+  int status[MAXK], its[MAXK];
+  unsigned long long bar;
+  int err, pad;
 };
 
 struct BcgPtrs {
@@ -90,155 +302,299 @@ struct BcgPtrs {
   double* r;
   double* p;
   double* y;
-  double* partials;  // [CTAs][MAXK]
+  double* partials;  // two arrays of [CTAs][MAXK]
   BcgState* st;
-  int64_t n;
-  int nrhs;
+  int nrhs, kmax;
+  double rtol2;
+  unsigned long long wait_ns;
 };
 
-// Per-column sums: thread t contributes v to column col (-1: nothing).  The
-// CTA's column sums go to partials[blockIdx.x][col] (threads in index order);
-// the last CTA to arrive sums each column's partials in CTA order.
-__device__ bool column_sums(double v, int col, const BcgPtrs& c, unsigned int* ticket,
-                            double* out /*[MAXK]*/) {
-  __shared__ double s[BBS];
-  __shared__ int sc[BBS];
-  __shared__ bool last;
-  s[threadIdx.x] = v;
-  sc[threadIdx.x] = col;
+struct BcgShared {
+  double red[CBS * 2];          // per-thread sums, V per thread
+  double part[CBS / 32][MAXK];  // per-warp sums of the partials
+  double tot[MAXK];
+  double rr0[MAXK], rr[MAXK], alpha[MAXK], beta[MAXK];
+  int active[MAXK], status[MAXK], its[MAXK];
+  int ok;
+};
+
+// Sum over the grid of every column's share: thread t holds V sums of columns
+// (t % stride) V .. + V - 1 (threads from `used` on hold none).  All threads
+// of every CTA get the totals in sh.tot, in the same fixed order: a CTA adds
+// its threads in index order by 32 lanes per column, publishes one partial
+// per column, and after the barrier every CTA adds all partials.
+template <int V>
+__device__ __forceinline__ bool column_sums(const double (&v)[V], int stride, int used,
+                                            const BcgPtrs& c, double* parts,
+                                            unsigned long long target, BcgShared& sh) {
+  const int tid = int(threadIdx.x), lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int i = 0; i < V; ++i) sh.red[tid * V + i] = v[i];
   __syncthreads();
-  if (threadIdx.x < MAXK) {
+  for (int col = warp; col < c.nrhs; col += CBS / 32) {
     double t = 0.0;
-    if (int(threadIdx.x) < c.nrhs)
-      for (int i = 0; i < BBS; ++i)
-        if (sc[i] == int(threadIdx.x)) t += s[i];
-    c.partials[blockIdx.x * MAXK + threadIdx.x] = t;
+    for (int q = col / V + lane * stride; q < used; q += 32 * stride)
+      t += sh.red[q * V + col % V];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) __stcg(parts + blockIdx.x * MAXK + col, t);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  if (tid == 0) sh.ok = grid_arrive_wait(&c.st->bar, target, &c.st->err, c.wait_ns);
+  __syncthreads();
+  if (!sh.ok) return false;
+  double t = 0.0;
+  if (lane < c.nrhs)
+    for (unsigned int b = warp; b < gridDim.x; b += CBS / 32) t += __ldcg(parts + b * MAXK + lane);
+  sh.part[warp][lane] = t;
+  __syncthreads();
+  if (tid < c.nrhs) {
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < CBS / 32; ++w) s += sh.part[w][tid];
+    sh.tot[tid] = s;
   }
   __syncthreads();
-  if (!last) return false;
-  __threadfence();
-  if (threadIdx.x < MAXK) {
-    double t = 0.0;
-    for (unsigned int b = 0; b < gridDim.x; ++b) t += __ldcg(c.partials + b * MAXK + threadIdx.x);
-    out[threadIdx.x] = t;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) *ticket = 0u;
   return true;
 }
 
-#define BCG_LOOP(i) \
-  for (int64_t i = blockIdx.x * int64_t(BBS) + threadIdx.x; i < c.n * c.nrhs; i += int64_t(gridDim.x) * BBS)
-
-// The elementwise kernels give thread t the entries t, t + G, ... with G a
-// multiple of nrhs (the grid stride), so a thread always sees the same
-// right-hand side col = t % nrhs.
-__global__ void __launch_bounds__(BBS) bcg_init(const BcgPtrs c, cudaGraphConditionalHandle h) {
-  __shared__ double tot[MAXK];
-  const int col = int((blockIdx.x * int64_t(BBS) + threadIdx.x) % c.nrhs);
-  double acc = 0.0;
-  BCG_LOOP(i) {
-    const double bi = c.b[i];
-    c.r[i] = bi;
-    c.p[i] = bi;
-    c.x[i] = 0.0;
-    acc += bi * bi;
-  }
-  if (column_sums(acc, col, c, &c.st->t0, tot) && threadIdx.x == 0) {
-    BcgState* st = c.st;
-    int any = 0;
-    for (int l = 0; l < c.nrhs; ++l) {
-      st->rr0[l] = tot[l];
-      st->rr[l] = tot[l];
-      st->active[l] = tot[l] > 0.0 && isfinite(tot[l]);
-      st->status[l] = SPMV_SUCCESS;
-      st->its[l] = 0;
-      any |= st->active[l];
+// One cooperative launch per solve.  Per iteration, on the CTA's rows:
+//   A  Y = A P, p.y                                  -> grid sum, alpha
+//   B  r -= alpha y, r.r                             -> grid sum, beta, tests
+//   C  x += alpha p, p = r + beta p                  -> grid barrier
+// (columns that have stopped are left as they are).
+template <int KL, class R>
+__global__ void __launch_bounds__(CBS)
+    bcg_kernel(const __grid_constant__ SpmvArgs a, const BcgPtrs c,
+               const RowChunks ch) {
+  // Right-hand sides per thread in the vector phases.
+  constexpr int V = R::SPLIT ? 1 : R::V;
+  using RV = Run<V, false>;
+  __shared__ BcgShared sh;
+  const int k = c.nrhs, tid = int(threadIdx.x);
+  // Vector phases: thread t takes runs of V entries t, t + used, ... of the
+  // CTA's chunks; used is a multiple of the runs per row, so its columns are
+  // fixed.
+  const int kv = k / V, used = CBS / kv * kv;
+  const RV vr(tid % kv, k);
+  const int c0 = vr.c0;
+  const int64_t step = int64_t(used) * V;
+  auto each = [&](auto&& body) {
+    if (tid < used)
+      for (int q = blockIdx.x; q < ch.count; q += gridDim.x) {
+        const int64_t e1 = ch.end(q) * k;
+#pragma unroll 2
+        for (int64_t e = ch.begin(q) * k + int64_t(tid) * V; e < e1; e += step) body(e);
+      }
+  };
+  unsigned long long epoch = 0;
+  double acc[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) acc[i] = 0.0;
+  each([&](int64_t e) {
+    double bv[V], z[V];
+    ld_run<double>(vr, c.b + e, bv);
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      z[i] = 0.0;
+      acc[i] += bv[i] * bv[i];
     }
-    st->k = 0;
-    cudaGraphSetConditional(h, (any && st->kmax > 0) ? 1u : 0u);
-  }
-}
-
-template <int K>
-__global__ void __launch_bounds__(BBS)
-    bcg_spmm_dot(const __grid_constant__ SpmvArgs a, const BcgPtrs c,
-                 cudaGraphConditionalHandle h) {
-  __shared__ double tot[MAXK];
-  if (blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(h, 0u);
-  double acc = 0.0;
-  // K lanes per row and BBS % K == 0, so this thread's lane (= column) is
-  // fixed: threadIdx.x % K.
-  spmm_rows<double, K>(a, c.nrhs, [&](const PartArg& P, int row, int lane, double v) {
-    static_cast<double*>(P.y)[int64_t(row) * c.nrhs + lane] = v;
-    acc += static_cast<const double*>(P.xown)[int64_t(row) * c.nrhs + lane] * v;
+    st_run<double>(vr, c.r + e, bv);
+    st_run<double>(vr, c.p + e, bv);
+    st_run<double>(vr, c.x + e, z);
   });
-  const int lane = int(threadIdx.x) % K;
-  if (column_sums(acc, lane < c.nrhs ? lane : -1, c, &c.st->t1, tot) && threadIdx.x == 0) {
-    BcgState* st = c.st;
-    for (int l = 0; l < c.nrhs; ++l) {
-      st->pap[l] = tot[l];
-      if (!st->active[l]) {
-        st->alpha[l] = 0.0;
-        continue;
+  // Consecutive sums publish into two arrays in turn: a CTA that runs ahead
+  // never overwrites partials another still reads.
+  auto parts = [&]() { return c.partials + (epoch & 1) * size_t(MAXK) * gridDim.x; };
+  ++epoch;
+  bool ok = column_sums<V>(acc, kv, used, c, parts(), epoch * gridDim.x, sh);
+  int go = 0;
+  if (tid < k) {
+    const double rr = sh.tot[tid];
+    sh.rr0[tid] = sh.rr[tid] = rr;
+    sh.alpha[tid] = sh.beta[tid] = 0.0;
+    sh.active[tid] = rr > 0.0 && isfinite(rr);
+    sh.status[tid] = SPMV_SUCCESS;
+    sh.its[tid] = 0;
+    go = sh.active[tid];
+  }
+  go = __syncthreads_or(go) && ok && c.kmax > 0;
+  for (int it = 1; go; ++it) {
+    // A.  A thread's right-hand sides follow from its lane: tid % KL.
+    double py[R::V];
+#pragma unroll
+    for (int i = 0; i < R::V; ++i) py[i] = 0.0;
+    for (int q = blockIdx.x; q < ch.count; q += gridDim.x)
+      spmm_rows<double, CBS, KL, R>(
+          a, k, ch.begin(q), ch.end(q),
+          [&](const PartArg& P, int row, const R& run, const double(&s)[R::V]) {
+            const int64_t o = int64_t(row) * k + run.c0;
+            double pv[R::V];
+            ld_run<double>(run, static_cast<const double*>(P.xown) + o, pv);
+            st_run<double>(run, static_cast<double*>(P.y) + o, s);
+#pragma unroll
+            for (int i = 0; i < R::V; ++i) py[i] += pv[i] * s[i];
+          });
+    ++epoch;
+    if (!column_sums<R::V>(py, KL, CBS, c, parts(), epoch * gridDim.x, sh)) break;
+    if (tid < k) {
+      double alpha = 0.0;
+      if (sh.active[tid]) {
+        const double pap = sh.tot[tid];
+        if (pap == 0.0 || !isfinite(pap)) {
+          sh.status[tid] = SPMV_ERROR_BREAKDOWN;
+          sh.active[tid] = 0;
+        } else {
+          alpha = sh.rr[tid] / pap;
+        }
       }
-      if (tot[l] == 0.0 || !isfinite(tot[l])) {
-        st->status[l] = SPMV_ERROR_BREAKDOWN;
-        st->active[l] = 0;
-        st->alpha[l] = 0.0;
+      sh.alpha[tid] = alpha;
+    }
+    __syncthreads();
+    // B.
+    double al[V], be[V];
+    bool act[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      act[i] = sh.active[c0 + i];
+      al[i] = sh.alpha[c0 + i];
+      acc[i] = 0.0;
+    }
+    each([&](int64_t e) {
+      double rv[V], yv[V];
+      ld_run<double>(vr, c.r + e, rv);
+      ld_run<double>(vr, c.y + e, yv);
+#pragma unroll
+      for (int i = 0; i < V; ++i)
+        if (act[i]) {
+          rv[i] = rv[i] - al[i] * yv[i];
+          acc[i] += rv[i] * rv[i];
+        }
+      st_run<double>(vr, c.r + e, rv);
+    });
+    ++epoch;
+    if (!column_sums<V>(acc, kv, used, c, parts(), epoch * gridDim.x, sh)) break;
+    go = 0;
+    // A column that stops in this iteration still takes C's x update.
+    if (tid < k) {
+      if (sh.active[tid]) {
+        const double rr = sh.tot[tid];
+        sh.its[tid] = it;
+        sh.beta[tid] = rr / sh.rr[tid];
+        sh.rr[tid] = rr;
+        if (rr / sh.rr0[tid] < c.rtol2) sh.active[tid] = 0;
       } else {
-        st->alpha[l] = st->rr[l] / tot[l];
+        sh.beta[tid] = 0.0;
       }
+      go = sh.active[tid] && it < c.kmax;
     }
+    go = __syncthreads_or(go);
+    // C.
+#pragma unroll
+    for (int i = 0; i < V; ++i) be[i] = sh.beta[c0 + i];
+    each([&](int64_t e) {
+      double xv[V], pv[V], rv[V];
+      ld_run<double>(vr, c.x + e, xv);
+      ld_run<double>(vr, c.p + e, pv);
+      ld_run<double>(vr, c.r + e, rv);
+#pragma unroll
+      for (int i = 0; i < V; ++i)
+        if (act[i]) {
+          xv[i] = xv[i] + al[i] * pv[i];
+          pv[i] = rv[i] + be[i] * pv[i];
+        }
+      st_run<double>(vr, c.x + e, xv);
+      st_run<double>(vr, c.p + e, pv);
+    });
+    if (!go) break;
+    ++epoch;
+    __syncthreads();
+    if (tid == 0) sh.ok = grid_arrive_wait(&c.st->bar, epoch * gridDim.x, &c.st->err, c.wait_ns);
+    __syncthreads();
+    if (!sh.ok) break;
+  }
+  if (blockIdx.x == 0 && tid < k) {
+    c.st->rr0[tid] = sh.rr0[tid];
+    c.st->rr[tid] = sh.rr[tid];
+    c.st->status[tid] = sh.status[tid];
+    c.st->its[tid] = sh.its[tid];
   }
 }
 
-__global__ void __launch_bounds__(BBS)
-    bcg_update_xr(const BcgPtrs c, cudaGraphConditionalHandle h) {
-  __shared__ double tot[MAXK];
-  const int col = int((blockIdx.x * int64_t(BBS) + threadIdx.x) % c.nrhs);
-  const BcgState* st = c.st;
-  const bool act = st->active[col];
-  const double alpha = st->alpha[col];
-  double acc = 0.0;
-  if (act) {
-    BCG_LOOP(i) {
-      c.x[i] = c.x[i] + alpha * c.p[i];
-      const double ri = c.r[i] - alpha * c.y[i];
-      c.r[i] = ri;
-      acc += ri * ri;
-    }
-  }
-  if (column_sums(acc, col, c, &c.st->t2, tot) && threadIdx.x == 0) {
-    BcgState* s = c.st;
-    s->k += 1;
-    int any = 0;
-    for (int l = 0; l < c.nrhs; ++l) {
-      if (!s->active[l]) {
-        s->beta[l] = 0.0;
-        continue;
-      }
-      s->its[l] = s->k;
-      s->beta[l] = tot[l] / s->rr[l];
-      s->rr[l] = tot[l];
-      if (tot[l] / s->rr0[l] < s->rtol2) s->active[l] = 0;
-      any |= s->active[l];
-    }
-    cudaGraphSetConditional(h, (any && s->k < s->kmax) ? 1u : 0u);
-  }
+// Lanes per row for k right-hand sides at v per lane.
+int lanes_for(int k, int v) {
+  int kl = 1;
+  while (kl * v < k) kl <<= 1;
+  return kl;
 }
 
-__global__ void __launch_bounds__(BBS) bcg_update_p(const BcgPtrs c) {
-  const int col = int((blockIdx.x * int64_t(BBS) + threadIdx.x) % c.nrhs);
-  // A column that converged in this iteration still had its beta set; one
-  // that was already inactive has beta 0 and p = r is harmless (unused).
-  const double beta = c.st->beta[col];
-  BCG_LOOP(i) c.p[i] = c.r[i] + beta * c.p[i];
+// Right-hand sides per lane: the widest run of at most 16 bytes that divides
+// k and to which every vector is aligned; two loaded one by one (0) when k is
+// odd or a vector is not aligned to two values.
+int run_width(int k, size_t es, int P, const void* const* x, const void* const* y) {
+  uintptr_t bits = 0;
+  for (int r = 0; r < P; ++r) bits |= reinterpret_cast<uintptr_t>(x[r]) |
+                                      reinterpret_cast<uintptr_t>(y[r]);
+  if (k == 1) return 1;
+  int v = int(16 / es);
+  while (v > 1 && (k % v != 0 || bits % (v * es) != 0)) v /= 2;
+  return v > 1 ? v : 0;
+}
+
+// Every row in one launch table (each rank's arrays; the CTAs' rows come from
+// the cut table).
+SpmvArgs spmm_args(spmv_matrix A, const int32_t* cols, size_t es, const void* const* x,
+                   void* const* y, const void* const* xown) {
+  SpmvArgs a;
+  fill_spmv_args(a, A->fwd, cols, es, x, y, xown, BBS, 1);
+  return a;
+}
+
+// Chunks of at most `most` rows, in whole rounds of `grid` CTAs (equal
+// shares).
+RowChunks row_chunks(spmv_matrix A, int grid, int64_t most) {
+  RowChunks ch{};
+  for (const DevPart& D : A->fwd.parts) ch.total += D.nrows;
+  const int64_t rounds = std::max<int64_t>(1, (ch.total + grid * most - 1) / (grid * most));
+  ch.rows = std::max<int64_t>(1, (ch.total + grid * rounds - 1) / (grid * rounds));
+  ch.count = int((ch.total + ch.rows - 1) / ch.rows);
+  return ch;
+}
+
+template <typename T, class R>
+const void* spmm_fn(int kl) {
+  switch (kl) {
+    case 1: return (const void*)spmm_kernel<T, 1, R>;
+    case 2: return (const void*)spmm_kernel<T, 2, R>;
+    case 4: return (const void*)spmm_kernel<T, 4, R>;
+    case 8: return (const void*)spmm_kernel<T, 8, R>;
+    case 16: if constexpr (R::V == 2) return (const void*)spmm_kernel<T, 16, R>;
+  }
+  fail(SPMV_ERROR_INTERNAL, "spmv: no block product for this width");
+}
+
+template <typename T>
+const void* spmm_walk_fn(int kl) {
+  switch (kl) {
+    case 2: return (const void*)spmm_walk_kernel<T, 2>;
+    case 4: return (const void*)spmm_walk_kernel<T, 4>;
+    case 8: return (const void*)spmm_walk_kernel<T, 8>;
+    case 16: return (const void*)spmm_walk_kernel<T, 16>;
+    case 32: return (const void*)spmm_walk_kernel<T, 32>;
+  }
+  fail(SPMV_ERROR_INTERNAL, "spmv: no block product for this width");
+}
+
+template <class R>
+const void* bcg_fn(int kl) {
+  switch (kl) {
+    case 1: return (const void*)bcg_kernel<1, R>;
+    case 2: return (const void*)bcg_kernel<2, R>;
+    case 4: return (const void*)bcg_kernel<4, R>;
+    case 8: return (const void*)bcg_kernel<8, R>;
+    case 16: return (const void*)bcg_kernel<16, R>;
+  }
+  fail(SPMV_ERROR_INTERNAL, "spmv: no block solver for this width");
 }
 
 }  // namespace
@@ -249,142 +605,115 @@ void launch_spmm(spmv_matrix A, int k, const void* const* x, void* const* y,
   require(k >= 1 && k <= MAXK, "spmv: block products take 1..32 right-hand sides");
   require(A->dtype == SPMV_FLOAT64 || A->dtype == SPMV_FLOAT32,
           "spmv: only float64 and float32 products are implemented");
-  int K = 1;
-  while (K < k) K <<= 1;
-  SpmvArgs a;
-  fill_spmv_args(a, A->fwd, A->fwd.cols.as<int32_t>(), dtype_size(A->dtype), x, y,
-                 nullptr, BBS / K, max_blocks_for(A->comm->num_sms, BBS));
-  if (a.nblocks == 0) return;
-#define SPMVB_SPMM(T)                                                             \
-  switch (K) {                                                                    \
-    case 1: spmm_kernel<T, 1><<<a.nblocks, BBS, 0, stream>>>(a, k); break;        \
-    case 2: spmm_kernel<T, 2><<<a.nblocks, BBS, 0, stream>>>(a, k); break;        \
-    case 4: spmm_kernel<T, 4><<<a.nblocks, BBS, 0, stream>>>(a, k); break;        \
-    case 8: spmm_kernel<T, 8><<<a.nblocks, BBS, 0, stream>>>(a, k); break;        \
-    case 16: spmm_kernel<T, 16><<<a.nblocks, BBS, 0, stream>>>(a, k); break;      \
-    default: spmm_kernel<T, 32><<<a.nblocks, BBS, 0, stream>>>(a, k); break;      \
+  const size_t es = dtype_size(A->dtype);
+  const int v = run_width(k, es, A->comm->size, x, y);
+  const bool f64 = A->dtype == SPMV_FLOAT64;
+  // Right-hand sides that cannot be loaded in aligned runs, on rows that take
+  // several batches: the tile walk, unless some row is for a whole CTA.
+  if (v == 0 && A->fwd.mean_row > SPMM_BATCH && A->fwd.max_row <= LONG_ROW) {
+    const int kl = lanes_for(k, 1);
+    SpmvArgs t;
+    fill_spmv_args(t, A->fwd, A->fwd.cols.as<int32_t>(), es, x, y, nullptr, BBS / kl,
+                   max_blocks_for(A->comm->num_sms, BBS));
+    if (t.nblocks == 0) return;
+    void* args[] = {&t, &k};
+    SPMVB_CUDA(cudaLaunchKernel(f64 ? spmm_walk_fn<double>(kl) : spmm_walk_fn<float>(kl),
+                                dim3(t.nblocks), dim3(BBS), args, 0, stream));
+    return;
   }
-  if (A->dtype == SPMV_FLOAT64) {
-    SPMVB_SPMM(double)
-  } else {
-    SPMVB_SPMM(float)
-  }
-#undef SPMVB_SPMM
-  SPMVB_CUDA(cudaGetLastError());
+  const SpmvArgs a = spmm_args(A, A->fwd.cols.as<int32_t>(), es, x, y, nullptr);
+  const int kl = lanes_for(k, v ? v : 2);
+  const void* fn;
+  if (k == 1)
+    fn = f64 ? (const void*)spmm_kernel<double, 1, Run<1, false>>
+             : (const void*)spmm_kernel<float, 1, Run<1, false>>;
+  else if (f64)
+    fn = v == 2 ? spmm_fn<double, Run<2, false>>(kl) : spmm_fn<double, Run<2, true>>(kl);
+  else
+    fn = v == 4   ? spmm_fn<float, Run<4, false>>(kl)
+         : v == 2 ? spmm_fn<float, Run<2, false>>(kl)
+                  : spmm_fn<float, Run<2, true>>(kl);
+  RowChunks ch = row_chunks(A, std::max(1, A->comm->num_sms) * BCPS,
+                            std::max(128, SPMM_CHUNK / k));
+  if (ch.count == 0) return;
+  void* args[] = {const_cast<SpmvArgs*>(&a), &ch, &k};
+  SPMVB_CUDA(cudaLaunchKernel(fn, dim3(ch.count), dim3(BBS), args, 0, stream));
 }
 
-// Block CG in the fused-halo layout over row-major n x k blocks; d_b, d_x
-// are global-layout device blocks.
-void block_cg(spmv_matrix A, int k, const double* d_b, double* d_x, int max_its,
-              double rtol, spmv_cg_info* info) {
-  require(k >= 1 && k <= MAXK, "spmv: block CG takes 1..32 right-hand sides");
+void destroy_block_workspace(BlockWorkspace* w) { delete w; }
+
+BlockWorkspace& block_workspace(spmv_matrix A, int k) {
+  if (!A->blk)
+    A->blk = std::unique_ptr<BlockWorkspace, void (*)(BlockWorkspace*)>(new BlockWorkspace,
+                                                                        destroy_block_workspace);
+  BlockWorkspace& w = *A->blk;
+  w.n = A->row_map->ranges.back();
+  const size_t bytes = sizeof(double) * std::max<int64_t>(w.n * k, 1);
+  for (DevBuf* v : {&w.b, &w.x, &w.r, &w.p, &w.y}) v->reserve(bytes);
+  w.state.reserve(sizeof(BcgState));
+  w.partials.reserve(sizeof(double) * 2 * MAXK * size_t(std::max(1, A->comm->num_sms)));
+  return w;
+}
+
+// Block CG in the fused-halo layout over the workspace's row-major n x k
+// blocks: w.b to w.x.
+void block_cg(spmv_matrix A, BlockWorkspace& w, int k, int max_its, double rtol,
+              spmv_cg_info* info) {
   spmv_comm comm = A->comm;
   build_global_cols(A);
-  const int64_t n = A->row_map->ranges.back();
   const int P = comm->size;
-  DevBuf r, p, y, partials, state;
-  const size_t bytes = sizeof(double) * std::max<int64_t>(n * k, 1);
-  r.reserve(bytes);
-  p.reserve(bytes);
-  y.reserve(bytes);
-  state.reserve(sizeof(BcgState));
-  SPMVB_CUDA(cudaMemset(state.ptr, 0, sizeof(BcgState)));
-  int K = 1;
-  while (K < k) K <<= 1;
   std::vector<const void*> xs(P), own(P);
   std::vector<void*> ys(P);
   for (int q = 0; q < P; ++q) {
     const int64_t off = A->row_map->ranges[q] * k;
-    xs[q] = p.as<double>();
-    own[q] = p.as<double>() + off;
-    ys[q] = y.as<double>() + off;
+    xs[q] = w.p.as<double>();
+    own[q] = w.p.as<double>() + off;
+    ys[q] = w.y.as<double>() + off;
   }
-  SpmvArgs a;
-  fill_spmv_args(a, A->fwd, A->fwd.cols_global.as<int32_t>(), sizeof(double), xs.data(),
-                 ys.data(), own.data(), BBS / K, max_blocks_for(comm->num_sms, BBS));
-  // Elementwise grid: a multiple of k threads so each thread keeps one column.
-  const int ew_threads = BBS;
-  int ew_grid = std::max(1, comm->num_sms) * (2048 / BBS);
-  while ((int64_t(ew_grid) * ew_threads) % k) ++ew_grid;
-  partials.reserve(sizeof(double) * MAXK * std::max(a.nblocks, ew_grid));
-  BcgPtrs c;
-  c.b = d_b;
-  c.x = d_x;
-  c.r = r.as<double>();
-  c.p = p.as<double>();
-  c.y = y.as<double>();
-  c.partials = partials.as<double>();
-  c.st = state.as<BcgState>();
-  c.n = n;
+  SpmvArgs a = spmm_args(A, A->fwd.cols_global.as<int32_t>(), sizeof(double), xs.data(),
+                         ys.data(), own.data());
+  BcgPtrs c{};
+  c.b = w.b.as<double>();
+  c.x = w.x.as<double>();
+  c.r = w.r.as<double>();
+  c.p = w.p.as<double>();
+  c.y = w.y.as<double>();
+  c.partials = w.partials.as<double>();
+  c.st = w.state.as<BcgState>();
   c.nrhs = k;
-  BcgState host{};
-  host.kmax = max_its;
-  host.nrhs = k;
-  host.rtol2 = rtol * rtol;
+  c.kmax = max_its;
+  c.rtol2 = rtol * rtol;
+  c.wait_ns = fused_wait_ns();
   cudaStream_t s = comm->stream;
-  SPMVB_CUDA(cudaMemcpyAsync(&c.st->k, &host.k, sizeof(int) * 4, cudaMemcpyHostToDevice, s));
-  SPMVB_CUDA(cudaMemcpyAsync(&c.st->rtol2, &host.rtol2, sizeof(double),
-                             cudaMemcpyHostToDevice, s));
-
-  using K1 = void (*)(SpmvArgs, BcgPtrs, cudaGraphConditionalHandle);
-  K1 k1;
-  switch (K) {
-    case 1: k1 = bcg_spmm_dot<1>; break;
-    case 2: k1 = bcg_spmm_dot<2>; break;
-    case 4: k1 = bcg_spmm_dot<4>; break;
-    case 8: k1 = bcg_spmm_dot<8>; break;
-    case 16: k1 = bcg_spmm_dot<16>; break;
-    default: k1 = bcg_spmm_dot<32>; break;
-  }
-  cudaGraph_t g = nullptr;
-  cudaGraphExec_t ge = nullptr;
-  cudaGraphConditionalHandle h;
-  SPMVB_CUDA(cudaGraphCreate(&g, 0));
-  try {
-    SPMVB_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
-    auto add = [&](cudaGraphNode_t* node, cudaGraph_t gg, const cudaGraphNode_t* dep,
-                   size_t nd, void* fn, int grid, void** args) {
-      cudaKernelNodeParams kp{};
-      kp.func = fn;
-      kp.gridDim = dim3(grid);
-      kp.blockDim = dim3(BBS);
-      kp.kernelParams = args;
-      SPMVB_CUDA(cudaGraphAddKernelNode(node, gg, dep, nd, &kp));
-    };
-    cudaGraphNode_t n0, nl, b1, b2, b3;
-    void* a0[] = {&c, &h};
-    add(&n0, g, nullptr, 0, (void*)bcg_init, ew_grid, a0);
-    cudaGraphNodeParams cp{};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    SPMVB_CUDA(cudaGraphAddNode(&nl, g, &n0, 1, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    void* a1[] = {&a, &c, &h};
-    add(&b1, body, nullptr, 0, (void*)k1, a.nblocks, a1);
-    void* a2[] = {&c, &h};
-    add(&b2, body, &b1, 1, (void*)bcg_update_xr, ew_grid, a2);
-    void* a3[] = {&c};
-    add(&b3, body, &b2, 1, (void*)bcg_update_p, ew_grid, a3);
-    SPMVB_CUDA(cudaGraphInstantiate(&ge, g, 0));
-    SPMVB_CUDA(cudaGraphLaunch(ge, s));
-    SPMVB_CUDA(cudaMemcpyAsync(&host, c.st, sizeof(BcgState), cudaMemcpyDeviceToHost, s));
-    SPMVB_CUDA(cudaStreamSynchronize(s));
-  } catch (...) {
-    if (ge) cudaGraphExecDestroy(ge);
-    cudaGraphDestroy(g);
-    throw;
-  }
-  soft_check(cudaGraphExecDestroy(ge), "cudaGraphExecDestroy");
-  soft_check(cudaGraphDestroy(g), "cudaGraphDestroy");
-  if (info)
-    for (int l = 0; l < k; ++l) {
-      info[l].iterations = host.its[l];
-      info[l].status = host.status[l];
-      info[l].rnorm0 = host.rr0[l];
-      info[l].rnorm = host.rr[l];
+  const int kl = lanes_for(k, 2);
+  const void* fn = k == 1       ? (const void*)bcg_kernel<1, Run<1, false>>
+                   : k % 2 == 0 ? bcg_fn<Run<2, false>>(kl)
+                                : bcg_fn<Run<2, true>>(kl);
+  // Every CTA resident; a device that cannot hold the grid at once (a context
+  // with fewer SMs) gets a smaller one.
+  int grid = std::max(1, comm->num_sms);
+  for (;;) {
+    SPMVB_CUDA(cudaMemsetAsync(c.st, 0, sizeof(BcgState), s));
+    RowChunks ch = row_chunks(A, grid, std::max(128, BCG_CHUNK / k));
+    void* args[] = {&a, &c, &ch};
+    const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(CBS), args, 0, s);
+    if (e != cudaErrorCooperativeLaunchTooLarge || grid == 1) {
+      SPMVB_CUDA(e);
+      break;
     }
+    (void)cudaGetLastError();
+    grid = (grid + 1) / 2;
+  }
+  BcgState host{};
+  SPMVB_CUDA(cudaMemcpyAsync(&host, c.st, sizeof(BcgState), cudaMemcpyDeviceToHost, s));
+  SPMVB_CUDA(cudaStreamSynchronize(s));
+  if (host.err) fail(SPMV_ERROR_CUDA, "spmv::cg - a bounded wait of the block solve timed out");
+  for (int l = 0; l < k; ++l) {
+    info[l].iterations = host.its[l];
+    info[l].status = host.status[l];
+    info[l].rnorm0 = host.rr0[l];
+    info[l].rnorm = host.rr[l];
+  }
 }
 
 }  // namespace spmvb
@@ -449,10 +778,7 @@ int spmv_cg_block(spmv_matrix A, int nrhs, spmv_memory memory, const double* con
     cudaStream_t s = comm->stream;
     spmv_l2gmap rm = A->row_map, cm = A->col_map;
     const int P = comm->size;
-    const int64_t n = rm->ranges.back();
-    DevBuf db, dxb;
-    db.reserve(sizeof(double) * std::max<int64_t>(n * nrhs, 1));
-    dxb.reserve(sizeof(double) * std::max<int64_t>(n * nrhs, 1));
+    BlockWorkspace& w = block_workspace(A, nrhs);
     const cudaMemcpyKind in = memory == SPMV_MEMORY_HOST ? cudaMemcpyHostToDevice
                                                          : cudaMemcpyDeviceToDevice;
     const cudaMemcpyKind outk = memory == SPMV_MEMORY_HOST ? cudaMemcpyDeviceToHost
@@ -461,18 +787,18 @@ int spmv_cg_block(spmv_matrix A, int nrhs, spmv_memory memory, const double* con
       const int64_t M = rm->rank[r].local_size;
       if (M == 0) continue;
       require(b[r] != nullptr, "spmv::cg - Error: b is NULL");
-      SPMVB_CUDA(cudaMemcpyAsync(db.as<double>() + rm->ranges[r] * nrhs, b[r],
+      SPMVB_CUDA(cudaMemcpyAsync(w.b.as<double>() + rm->ranges[r] * nrhs, b[r],
                                  sizeof(double) * M * nrhs, in, s));
     }
     std::vector<spmv_cg_info> local(nrhs);
-    block_cg(A, nrhs, db.as<double>(), dxb.as<double>(), max_its, rtol, local.data());
+    block_cg(A, w, nrhs, max_its, rtol, local.data());
     for (int r = 0; r < P; ++r) {
       const int64_t M = rm->rank[r].local_size;
       const int64_t G = int64_t(cm->rank[r].ghosts.size());
       if (M + G == 0) continue;
       require(x[r] != nullptr, "spmv::cg - Error: x is NULL");
       if (M > 0)
-        SPMVB_CUDA(cudaMemcpyAsync(x[r], dxb.as<double>() + rm->ranges[r] * nrhs,
+        SPMVB_CUDA(cudaMemcpyAsync(x[r], w.x.as<double>() + rm->ranges[r] * nrhs,
                                    sizeof(double) * M * nrhs, outk, s));
       if (G > 0) {
         if (memory == SPMV_MEMORY_HOST)

@@ -274,6 +274,7 @@ struct DevCsr {
 
 struct CgWorkspace;  // cg.cu
 struct IrWorkspace;  // ir.cu
+struct BlockWorkspace;  // block.cu
 
 struct spmv_matrix_s {
   spmv_comm comm = nullptr;
@@ -297,6 +298,7 @@ struct spmv_matrix_s {
   bool kernel_set = false;
   std::unique_ptr<CgWorkspace, void (*)(CgWorkspace*)> cg{nullptr, nullptr};
   std::unique_ptr<IrWorkspace, void (*)(IrWorkspace*)> ir{nullptr, nullptr};
+  std::unique_ptr<BlockWorkspace, void (*)(BlockWorkspace*)> blk{nullptr, nullptr};
 };
 
 namespace spmvb {
@@ -486,13 +488,10 @@ void copy_rhs_in(spmv_matrix A, spmv_memory memory, const double* const* b, doub
 void copy_solution_out(spmv_matrix A, spmv_memory memory, const double* dx,
                        double* const* x);
 
-// Multi-right-hand-side product and block CG (block.cu); blocks are row-major
-// with leading dimension k.
+// Multi-right-hand-side product (block.cu); blocks are row-major with leading
+// dimension k.
 void launch_spmm(spmv_matrix A, int k, const void* const* x, void* const* y,
                  cudaStream_t stream);
-void block_cg(spmv_matrix A, int k, const double* d_b, double* d_x, int max_its,
-              double rtol, spmv_cg_info* info);
-
 
 
 // out[r][k] = scale * lambda[r][row(k)] * x[r][col(k)] (adjoint.cu).
