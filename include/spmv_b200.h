@@ -324,7 +324,8 @@ int spmv_matrix_solver_product(spmv_matrix A, int solver, spmv_kernel* kernel,
  * one cooperative launch per solve with *ctas_per_sm persistent CTAs per SM
  * and the residual held in shared memory (*r_shared = 1) or global memory,
  * 2 for the same launch in the merged-update form (two grid syncs per
- * iteration instead of three).
+ * iteration instead of three); *r_shared = 2: its on-chip form, p in shared
+ * memory and the residual in tensor memory.
  * Fails when spmv_cg has not run on the matrix.  No reference counterpart. */
 int spmv_matrix_cg_form(spmv_matrix A, int* fused, int* ctas_per_sm, int* r_shared);
 

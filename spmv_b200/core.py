@@ -347,8 +347,8 @@ class Matrix:
     def cg_form(self, solver="cg"):
         """How cg (solver="cg") or cg_mixed (solver="mixed") runs on this
         matrix: ("graph", 0, None) for its kernels in a CUDA graph, or
-        ("fused", CTAs per SM, "smem" or "global": where the residual lives)
-        for one cooperative launch per solve, with ":m" appended for cg's
+        ("fused", CTAs per SM, "smem", "tmem" or "global": where the residual
+        lives) for one cooperative launch per solve, with ":m" appended for cg's
         merged-update form (two grid syncs per iteration); fails if that
         solver has not run on the matrix."""
         fn = {"cg": "spmv_matrix_cg_form", "mixed": "spmv_matrix_cg_mixed_form"}[solver]
@@ -356,7 +356,7 @@ class Matrix:
         call(fn, self._h, C.byref(f), C.byref(cps), C.byref(rs))
         if not f.value:
             return "graph", 0, None
-        where = "smem" if rs.value else "global"
+        where = ("global", "smem", "tmem")[rs.value]
         return "fused", cps.value, where + (":m" if f.value == 2 else "")
 
     def get_kernel(self):

@@ -999,7 +999,7 @@ int spmv_matrix_cg_form(spmv_matrix A, int* fused, int* ctas_per_sm, int* r_shar
     const CgForm f = cg_form(A);
     *fused = f.fused ? (f.merged ? 2 : 1) : 0;
     *ctas_per_sm = f.cps;
-    *r_shared = f.rs ? 1 : 0;
+    *r_shared = f.tmem ? 2 : f.rs ? 1 : 0;
   });
 }
 

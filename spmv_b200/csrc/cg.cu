@@ -33,10 +33,11 @@
 // the product gathers it, saves K3's pass over p and r but doubles the
 // gathers; measured on the 7-point stencil it was slower.)
 //
-// With a staged product the whole solve can instead run as one cooperative
-// launch (cg_fused below: the same three phases per iteration separated by
-// grid barriers, the residual held in shared memory); the workspace times
-// both forms on the matrix and keeps the faster.
+// The whole solve can instead run as one cooperative launch: with its vectors
+// in shared and tensor memory (cg_onchip below) or, with a staged product, the
+// same three phases per iteration separated by grid barriers and the residual
+// in shared memory (cg_fused below); the workspace times what fits on the
+// matrix and keeps the fastest.
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
@@ -45,6 +46,7 @@
 #include <type_traits>
 
 #include "internal.h"
+#include "sell_ring.cuh"
 #include "sell_staged.cuh"
 #include "spmv_kernel.cuh"
 
@@ -64,6 +66,8 @@ struct CgWorkspace {
   int fused_grid = 0, fused_block = 0, fused_smem = 0, fused_cps = 0;
   bool fused_rs = false;
   bool fused_mg = false;  // the merged-update form
+  bool fused_tm = false;  // its on-chip form (r, y in tensor memory)
+  spmvb::OnchipShape onchip;
   spmvb::DevBuf bar, partials2, ctas;
   spmvb::SpmvArgs fused_args;
   const spmvb::StagedDesc* tiles = nullptr;
@@ -305,6 +309,44 @@ struct FusedScalars {
   int kmax, k, status, go;
 };
 
+// The final state (one thread).
+__device__ __forceinline__ void store_scalars(CgState* st, const FusedScalars& sv) {
+  st->rnorm0 = sv.rnorm0;
+  st->rnorm_old = sv.rnorm_old;
+  st->rnorm_new = sv.rnorm_new;
+  st->alpha = sv.alpha;
+  st->beta = sv.beta;
+  st->pdoty = sv.pdoty;
+  st->k = sv.k;
+  st->status = sv.status;
+}
+
+// The merged-update form's stopping test, alpha and beta from iteration k's
+// totals p.y, r.y, y.y, r.r (one thread; every CTA computes the same).
+__device__ __forceinline__ void merged_scalars(FusedScalars& sv, const double (&tot)[4], int k) {
+  const double rr = tot[3];
+  if (k > 0) {
+    sv.rnorm_new = rr;
+    sv.rnorm_old = rr;
+  }
+  if ((k > 0 && rr / sv.rnorm0 < sv.rtol2) || k >= sv.kmax) {
+    sv.go = false;
+    return;
+  }
+  const double py = tot[0];
+  sv.k = k + 1;
+  sv.pdoty = py;
+  sv.alpha = rr / py;
+  if (py == 0.0 || !isfinite(py)) {
+    sv.status = SPMV_ERROR_BREAKDOWN;
+    sv.go = false;
+    return;
+  }
+  const double a = sv.alpha;
+  const double rr1 = rr - 2.0 * a * tot[1] + a * a * tot[2];
+  sv.beta = rr1 / rr;
+}
+
 // The fused solve after its CTA's set-up, for the NT consumer threads (the
 // CTA's first NT): init, then per iteration phase A = product(k) (this
 // thread's share of p.y after y = A p over the CTA's rows), B and C with the
@@ -442,17 +484,7 @@ __device__ __forceinline__ bool cg_fused_solve(const CgPtrs& c, const FusedCta& 
       break;
     }
   }
-  if (tid == 0 && ok && blockIdx.x == 0) {
-    CgState* st = c.st;
-    st->rnorm0 = sv.rnorm0;
-    st->rnorm_old = sv.rnorm_old;
-    st->rnorm_new = sv.rnorm_new;
-    st->alpha = sv.alpha;
-    st->beta = sv.beta;
-    st->pdoty = sv.pdoty;
-    st->k = sv.k;
-    st->status = sv.status;
-  }
+  if (tid == 0 && ok && blockIdx.x == 0) store_scalars(c.st, sv);
   return ok;
 }
 
@@ -518,29 +550,7 @@ __device__ __forceinline__ bool cg_fused_solve_merged(const CgPtrs& c, const Fus
     }
     // The stopping test, alpha and beta (one thread; every CTA computes the
     // same from the same totals).
-    if (tid == 0) {
-      const double rr = tot[3];
-      if (k > 0) {
-        sv.rnorm_new = rr;
-        sv.rnorm_old = rr;
-      }
-      if ((k > 0 && rr / sv.rnorm0 < sv.rtol2) || k >= sv.kmax) {
-        sv.go = false;
-      } else {
-        const double py = tot[0];
-        sv.k = k + 1;
-        sv.pdoty = py;
-        sv.alpha = rr / py;
-        if (py == 0.0 || !isfinite(py)) {
-          sv.status = SPMV_ERROR_BREAKDOWN;
-          sv.go = false;
-        } else {
-          const double a = sv.alpha;
-          const double rr1 = rr - 2.0 * a * tot[1] + a * a * tot[2];
-          sv.beta = rr1 / rr;
-        }
-      }
-    }
+    if (tid == 0) merged_scalars(sv, tot, k);
     named_sync(1, NT);
     if (!sv.go) break;
 
@@ -581,17 +591,7 @@ __device__ __forceinline__ bool cg_fused_solve_merged(const CgPtrs& c, const Fus
     }
     ++k;
   }
-  if (tid == 0 && ok && blockIdx.x == 0) {
-    CgState* st = c.st;
-    st->rnorm0 = sv.rnorm0;
-    st->rnorm_old = sv.rnorm_old;
-    st->rnorm_new = sv.rnorm_new;
-    st->alpha = sv.alpha;
-    st->beta = sv.beta;
-    st->pdoty = sv.pdoty;
-    st->k = sv.k;
-    st->status = sv.status;
-  }
+  if (tid == 0 && ok && blockIdx.x == 0) store_scalars(c.st, sv);
   return ok;
 }
 
@@ -651,6 +651,245 @@ __global__ void __launch_bounds__(CFG::BS, CFG::MINB)
   if (tid == 0) pipe.stop = 1;
 }
 
+// ---------------------------------------------------------------------------
+// The merged-update solve with its vectors on chip.  What bounds the forms
+// above is the traffic between L2 and the SMs (7-point 128^3: about 417 MB
+// per iteration at 10.7 TB/s, of which the matrix is 146 MB): the gathers of p
+// and the vector phases' y, p, x, r.  Here each CTA keeps its rows' p in
+// shared memory, where most gathers of a banded matrix land, and r, y (and x,
+// when it fits) in tensor memory, each entry in the columns of the lane that
+// owns the row: only p (for the other CTAs' gathers) and x cross L2.  A warp
+// keeps the same slices in every phase and streams their entries through its
+// own ring (sell_ring.cuh).
+//
+// Measured (us per iteration; the form the workspace chose before): 7-point
+// 128^3 over 8 ranks 37.4 (42.3), of which the product takes 25 (the matrix at
+// 5.8 TB/s), the sum 4, the update 6 (x and p through L2) and the barrier 1.5;
+// 96^3 18.3 (22.3); 5-point 1024^2, x in tensor memory, 14.8 (20.3), product 7.6;
+// 48^3 and below 6.3 to 6.7 (17 to 20 as a CUDA graph): there the two syncs
+// (2.9 + 1.4) are most of it.
+template <int NW, int U, int D, int S, bool LATE, bool D16>
+__global__ void __launch_bounds__(NW * 32, 1)
+    cg_onchip(const __grid_constant__ OnchipShape o, const __grid_constant__ CgPtrs c,
+              const FusedCta* __restrict__ ctas) {
+  using CI = typename std::conditional<D16, int16_t, int32_t>::type;
+  using Shape = RingShape<double, CI, U, D, S>;
+  constexpr int NT = NW * 32;
+  extern __shared__ __align__(128) unsigned char staged_smem[];
+  __shared__ __align__(8) uint64_t bars[NW * D];
+  __shared__ GridTotals<NT, 4> g4;
+  __shared__ GridSum<NT> gs;
+  __shared__ FusedScalars sv;
+  __shared__ FusedCta me;
+  __shared__ uint32_t tm_base;
+  // Each lane's share of r.r from the update to the next product's sums.
+  __shared__ double rr_part[NT];
+  const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+  // Dynamic shared memory: the warps' slots, the CTA's item table, its p.
+  int4* const items = reinterpret_cast<int4*>(staged_smem + NW * Shape::BYTES);
+  double* const ps = reinterpret_cast<double*>(items + o.per_warp * NW);
+  if (tid == 0) me = ctas[blockIdx.x];
+  if (lane == 0) ring_init<D>(bars + warp * D);
+  if (warp == 0) tmem_alloc(&tm_base, uint32_t(o.alloc));
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  for (int j = tid; j < me.t1 - me.t0; j += NT) items[j] = __ldg(o.items + me.t0 + j);
+  __syncthreads();
+  // This warp's columns: its item i's slice q at tm + (i * S + q) * o.cols,
+  // r, y, x.
+  const uint32_t tm = tm_base + (uint32_t(warp & 3) << 21) +
+                      uint32_t((warp >> 2) * o.per_warp * S * o.cols);
+  auto view = [&]() {
+    return RingView<double, CI>{o.vals, static_cast<const CI*>(o.idx), items, me.t1 - me.t0, NW,
+                                staged_smem + warp * Shape::BYTES, bars + warp * D};
+  };
+  RingState ring;
+  ring_prime<double, CI, U, D, S>(view(), ring);
+  // The warp's items: body(rows, column of the item's first slice).
+  auto each_item = [&](auto&& body) {
+    const int n = me.t1 - me.t0;
+    uint32_t t = tm;
+    for (int j = warp; j < n; j += NW, t += S * o.cols) body(RingRows<S>(items[j]), t);
+  };
+
+  // Init: r = p = b, x = 0, rr_0 = b.b.
+  double rr = 0.0;
+  {
+    const uint64_t keep = l2_policy_keep();
+    each_item([&](const RingRows<S>& row, uint32_t t) {
+#pragma unroll
+      for (int q = 0; q < S; ++q) {
+        const int g = row.g[q];
+        const double bi = row.valid[q] ? c.b[g] : 0.0;
+        __syncwarp();
+        tmem_st(t + q * o.cols, bi);
+        if (o.cols == 6) tmem_st(t + q * o.cols + 4, 0.0);
+        if (row.valid[q]) {
+          ps[g - me.g0] = bi;
+          st_pol(c.p + g, bi, keep);
+          if (o.cols != 6) st_pol(c.x + g, 0.0, keep);
+          rr += bi * bi;
+        }
+      }
+    });
+    __syncwarp();
+    tmem_wait_st();
+  }
+  rr_part[tid] = rr;
+  // Barrier epochs: 1 for the init, 2k + 2 for iteration k's sum and 2k + 3 for
+  // its closing barrier.
+  double tot[4] = {rr, 0.0, 0.0, 0.0};
+  bool ok = coop_grid_totals<NT, 4>(tot, c.partials, c.bar, gridDim.x, &c.st->stage_err, c.wait_ns,
+                                   g4, tot);
+  const double rnorm0 = tot[0];
+  if (tid == 0) {
+    sv.rtol2 = *static_cast<volatile double*>(&c.st->rtol2);
+    sv.kmax = *static_cast<volatile int*>(&c.st->kmax);
+    sv.rnorm0 = sv.rnorm_old = sv.rnorm_new = rnorm0;
+    sv.alpha = sv.beta = sv.pdoty = 0.0;
+    sv.k = 0;
+    sv.status = SPMV_SUCCESS;
+    sv.go = ok && sv.kmax > 0 && rnorm0 > 0.0 && isfinite(rnorm0);
+  }
+  named_sync(1, NT);
+  int k = 0;
+  while (sv.go) {
+    // A: y = A p, the four sums.
+    double in[4] = {0.0, 0.0, 0.0, 0.0};
+    {
+      const uint64_t keep = l2_policy_keep();
+      const unsigned rows = unsigned(me.g1 - me.g0);
+      const int g0 = me.g0;
+      if (!ring_pass<double, CI, U, D, S, LATE>(
+              view(), ring,
+              [&](int col) {
+                const unsigned l = unsigned(col - g0);
+                return l < rows ? ps[l] : ld_pol(c.p + col, keep);
+              },
+              [&](int i, const RingRows<S>& row, const double(&sum)[S]) {
+                const uint32_t t = tm + i * S * o.cols;
+                Tmem64 rv[S];
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < S; ++q) {
+                  tmem_ld(t + q * o.cols, rv[q]);
+                  tmem_st(t + q * o.cols + 2, sum[q]);
+                }
+                tmem_wait_ld();
+#pragma unroll
+                for (int q = 0; q < S; ++q) {
+                  if (row.valid[q]) {
+                    in[0] += ps[row.g[q] - g0] * sum[q];
+                    in[1] += rv[q].get() * sum[q];
+                    in[2] += sum[q] * sum[q];
+                  }
+                }
+              }))
+        if (lane == 0) atomicExch(&c.st->stage_err, 1);
+      __syncwarp();
+      tmem_wait_st();
+    }
+    in[3] = rr_part[tid];
+    // (Two arrays of partials in turn: the init's may still be read when the
+    // first iteration's are published.)
+    if (!coop_grid_totals<NT, 4>(in, k == 0 ? c.partials + 4 * gridDim.x : c.partials, c.bar,
+                                (2ull * unsigned(k) + 2) * gridDim.x, &c.st->stage_err,
+                                c.wait_ns, g4, tot)) {
+      ok = false;
+      break;
+    }
+    if (tid == 0) merged_scalars(sv, tot, k);
+    named_sync(1, NT);
+    if (!sv.go) break;
+
+    // C: r -= alpha y, x += alpha p, p = p beta + r, this CTA's r.r.
+    {
+      const double alpha = sv.alpha, beta = sv.beta;
+      const uint64_t keep = l2_policy_keep();
+      const int g0 = me.g0;
+      const bool xt = o.cols == 6;
+      rr = 0.0;
+      // Two slices in flight per warp (the loads of both before
+      // the results of the first are needed).
+      const int n = me.t1 - me.t0;
+      constexpr int B = S == 1 ? 2 : 1;
+      uint32_t t = tm;
+      for (int j = warp; j < n; j += B * NW, t += B * S * o.cols) {
+        Tmem64 rv[B][S], yv[B][S], xv[B][S];
+        double xg[B][S];
+        RingRows<S> row[B];
+#pragma unroll
+        for (int h = 0; h < B; ++h) row[h] = RingRows<S>(items[min(j + h * NW, n - 1)]);
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < B; ++h)
+          if (h == 0 || j + NW < n)
+#pragma unroll
+            for (int q = 0; q < S; ++q) {
+              const uint32_t tq = t + (h * S + q) * o.cols;
+              tmem_ld(tq, rv[h][q]);
+              tmem_ld(tq + 2, yv[h][q]);
+              if (xt)
+                tmem_ld(tq + 4, xv[h][q]);
+              else if (row[h].valid[q])
+                xg[h][q] = ld_pol(c.x + row[h].g[q], keep);
+            }
+        __syncwarp();
+        tmem_wait_ld();
+#pragma unroll
+        for (int h = 0; h < B; ++h)
+          if (h == 0 || j + NW < n)
+#pragma unroll
+            for (int q = 0; q < S; ++q) {
+              const uint32_t tq = t + (h * S + q) * o.cols;
+              const int g = row[h].g[q];
+              const bool valid = row[h].valid[q];
+              const double pv = valid ? ps[g - g0] : 0.0;
+              const double ri = rv[h][q].get() - alpha * yv[h][q].get();
+              __syncwarp();
+              tmem_st(tq, ri);
+              if (xt) tmem_st(tq + 4, xv[h][q].get() + alpha * pv);
+              if (valid) {
+                const double pn = pv * beta + ri;
+                ps[g - g0] = pn;
+                st_pol(c.p + g, pn, keep);
+                if (!xt) st_pol(c.x + g, xg[h][q] + alpha * pv, keep);
+                rr += ri * ri;
+              }
+            }
+      }
+      __syncwarp();
+      tmem_wait_st();
+      rr_part[tid] = rr;
+    }
+    if (!coop_grid_barrier<NT>(c.bar, (2ull * unsigned(k) + 3) * gridDim.x, &c.st->stage_err,
+                               c.wait_ns, gs)) {
+      ok = false;
+      break;
+    }
+    ++k;
+  }
+  if (o.cols == 6)
+    each_item([&](const RingRows<S>& row, uint32_t t) {
+#pragma unroll
+      for (int q = 0; q < S; ++q) {
+        Tmem64 xv;
+        __syncwarp();
+        tmem_ld(t + q * o.cols + 4, xv);
+        tmem_wait_ld();
+        if (row.valid[q]) c.x[row.g[q]] = xv.get();
+      }
+    });
+  if (tid == 0 && ok && blockIdx.x == 0) store_scalars(c.st, sv);
+  ring_drain<double, CI, D>(view(), ring);
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (warp == 0) tmem_free(tm_base, uint32_t(o.alloc));
+}
+
 using FusedFn = void (*)(SpmvArgs, CgPtrs, const FusedCta*);
 
 // Fused shapes: one CTA per SM (28 consumer warps, 6 stages) or two
@@ -678,6 +917,37 @@ FusedFn fused_fn(const SolverProduct& sp) {
   return sp.d16 ? fused_fn_u<CFG, true, RS, MG>(sp.w) : fused_fn_u<CFG, false, RS, MG>(sp.w);
 }
 
+
+using OnchipFn = void (*)(OnchipShape, CgPtrs, const FusedCta*);
+
+// A kernel of the on-chip form and the bytes of its rings.
+struct OnchipKernel {
+  const void* fn;
+  int64_t ring_bytes;
+  int warps, slices;  // per CTA; slices per item
+};
+template <int NW, int U, int D, int S, bool LATE>
+OnchipKernel onchip_kernel(bool d16) {
+  if (d16)
+    return {(const void*)cg_onchip<NW, U, D, S, LATE, true>,
+            NW * int64_t(RingShape<double, int16_t, U, D, S>::BYTES), NW, S};
+  // (With 32-bit columns the early form of seven columns spills.)
+  return {(const void*)cg_onchip<NW, U, D, S, LATE || U == 7, false>,
+          NW * int64_t(RingShape<double, int32_t, U, D, S>::BYTES), NW, S};
+}
+// The kernels for a product, most warps first (the first that fits is used).
+std::vector<OnchipKernel> onchip_kernels(spmv_matrix A) {
+  const bool d = A->fwd.d16;
+  const int64_t w = A->fwd.max_row;
+  // Rows of at most 5 entries: pairs of slices (an item of one is mostly
+  // overhead: 1024^2 5-point, 20.0 us per iteration against 15.6).  At 7
+  // entries pairs gain nothing (128^3: 40.0 us against 42.7).  Wider rows: four
+  // columns a copy (rows of 13 to 25 entries, 216k rows: 15.8 us against 18.2
+  // with eight).
+  if (w <= 5) return {onchip_kernel<20, 5, 2, 2, true>(d), onchip_kernel<16, 5, 2, 2, false>(d)};
+  if (w <= 7) return {onchip_kernel<24, 7, 2, 1, true>(d), onchip_kernel<20, 7, 2, 1, false>(d)};
+  return {onchip_kernel<24, 4, 3, 1, false>(d), onchip_kernel<16, 4, 3, 1, false>(d)};
+}
 
 using K1Fn = void (*)(SpmvArgs, CgPtrs, cudaGraphConditionalHandle);
 
@@ -866,6 +1136,51 @@ bool plan_fused(spmv_matrix A, const SolverProduct& sp, FusedPlan& plan) {
   return true;
 }
 
+// The on-chip form: one CTA per SM; false when the CTAs' rows of p do not fit
+// beside the rings in shared memory, or their r and y in tensor memory.
+bool plan_onchip(spmv_matrix A, FusedPlan& plan) {
+  spmv_comm comm = A->comm;
+  const int grid = std::max(1, comm->num_sms);
+  for (const OnchipKernel& kn : onchip_kernels(A)) {
+    const ItemTable& t = item_table(A, kn.slices);
+    if (!t.ok) return false;
+    std::vector<FusedCta> ctas(static_cast<size_t>(grid));
+    const int64_t N = t.nitems;
+    int64_t rows = 0, items = 0;
+    for (int b = 0; b < grid; ++b) {
+      FusedCta& f = ctas[size_t(b)];
+      f.t0 = int32_t(N * b / grid);
+      f.t1 = int32_t(N * (b + 1) / grid);
+      f.g0 = t.row[size_t(f.t0)];
+      f.g1 = t.row[size_t(f.t1)];
+      rows = std::max<int64_t>(rows, f.g1 - f.g0);
+      items = std::max<int64_t>(items, f.t1 - f.t0);
+    }
+    OnchipShape o{};
+    o.vals = A->fwd.sell_vals.as<double>();
+    o.idx = A->fwd.d16 ? A->fwd.sell_d16_global.ptr : A->fwd.sell_cols_global.ptr;
+    o.items = t.desc.as<int4>();
+    const int64_t per_warp = (items + kn.warps - 1) / kn.warps;
+    for (int cols : {6, 4})
+      if (o.cols == 0 && per_warp * (kn.warps / 4) * kn.slices * cols <= 512) o.cols = cols;
+    if (o.cols == 0) continue;
+    o.per_warp = int(per_warp);
+    o.alloc = 32;
+    while (o.alloc < per_warp * (kn.warps / 4) * kn.slices * o.cols) o.alloc *= 2;
+    const int64_t smem = kn.ring_bytes + per_warp * kn.warps * int64_t(sizeof(int4)) +
+                         (rows * 8 + 15) / 16 * 16;
+    if (!fused_fits(comm, kn.fn, kn.warps * 32, 1, smem, plan)) continue;
+    plan.cps = 1;
+    plan.grid = grid;
+    plan.rs = true;
+    plan.merged = plan.tmem = true;
+    plan.ctas = std::move(ctas);
+    plan.onchip = o;
+    return true;
+  }
+  return false;
+}
+
 void use_plan(CgWorkspace& w, FusedPlan& plan) {
   w.fused = true;
   w.fused_fn = plan.fn;
@@ -875,10 +1190,13 @@ void use_plan(CgWorkspace& w, FusedPlan& plan) {
   w.fused_cps = plan.cps;
   w.fused_rs = plan.rs;
   w.fused_mg = plan.merged;
+  w.fused_tm = plan.tmem;
+  if (plan.tmem) w.onchip = plan.onchip;
   // One partial per CTA in each reduction's array (four in partials for the
-  // merged form).  partials is baked into the graph form's kernels and never
+  // merged form, twice four for its on-chip form).  partials is baked into the graph form's kernels and never
   // reallocated: it was sized for more CTAs than any plan has.
-  require(w.partials.bytes >= sizeof(double) * size_t(plan.grid) * (plan.merged ? 4 : 1),
+  require(w.partials.bytes >= sizeof(double) * size_t(plan.grid) *
+                                     (plan.tmem ? 8 : plan.merged ? 4 : 1),
           "spmv: fused CG grid larger than its partials array");
   w.partials2.reserve(sizeof(double) * size_t(plan.grid));
   w.ctas.reserve(sizeof(FusedCta) * plan.ctas.size());
@@ -895,12 +1213,12 @@ void enqueue_solve(CgWorkspace& w, cudaStream_t s) {
   if (w.fused) {
     const size_t g = size_t(w.fused_grid);
     require(w.partials.bytes >= g * sizeof(double) && w.partials2.bytes >= g * sizeof(double) &&
-                w.ctas.bytes >= g * sizeof(FusedCta) && w.tiles != nullptr,
+                w.ctas.bytes >= g * sizeof(FusedCta) && (w.fused_tm || w.tiles != nullptr),
             "spmv: fused CG buffers smaller than its grid");
     SPMVB_CUDA(cudaMemsetAsync(w.bar.ptr, 0, sizeof(unsigned long long), s));
     CgPtrs c = cg_ptrs(w);
     const FusedCta* ctas = w.ctas.as<FusedCta>();
-    void* args[] = {&w.fused_args, &c, &ctas};
+    void* args[] = {w.fused_tm ? (void*)&w.onchip : (void*)&w.fused_args, &c, &ctas};
     const cudaError_t e = cudaLaunchCooperativeKernel(
         w.fused_fn, dim3(w.fused_grid), dim3(w.fused_block), args, size_t(w.fused_smem), s);
     if (e != cudaErrorCooperativeLaunchTooLarge) {
@@ -950,18 +1268,19 @@ float time_iterations(CgWorkspace& w, cudaStream_t s, int its) {
 }
 
 // Chooses between the graph form and the fused plans that fit, by timing 32
-// iterations of each on b = 1 (the fused form needs a staged product):
+// iterations of each on b = 1: the on-chip form where its vectors fit, else
+// (with a staged product)
 // r in shared memory with one or two CTAs per SM (when the CTAs' rows fit),
 // or r in global memory with two CTAs of 6 stages or three of 4; and the
 // merged-update form (two grid syncs per iteration) of the 2-CTA shared and
 // 3-CTA global plans, whose one extra product per solve weighs 1/32 here.
 // SPMV_B200_CG_FUSED: "0" keeps the graph form; "<cps>:<smem|global>[:m]"
 // forces that plan (1:smem, 2:smem, 1:global, 2:global, 3:global, 2:smem:m,
-// 3:global:m), failing if it does not fit.
+// 3:global:m, and 1:tmem:m for the on-chip form), failing if it does not fit.
 void choose_form(spmv_matrix A, CgWorkspace& w) {
   w.fused = false;
   const SolverProduct& sp = w.product;
-  if (sp.kind != ProductKind::Staged || w.n == 0) return;
+  if (w.n == 0) return;
   const char* env = std::getenv("SPMV_B200_CG_FUSED");
   const std::string mode = env ? env : "";
   if (mode == "0") return;
@@ -969,18 +1288,27 @@ void choose_form(spmv_matrix A, CgWorkspace& w) {
   int coop = 0;
   SPMVB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, comm->device));
   if (!coop) return;
-  // The fused kernel streams the product's tile table.
-  const DevCsr::StagedTable& tiles = cg_tiles(A, sp);
-  if (!tiles.ok) return;
-  w.tiles = tiles.desc.as<StagedDesc>();
-  w.ntiles = tiles.ntiles;
+  // The on-chip form walks the SELL slices itself, whatever K1's product; a
+  // kernel set on the matrix other than the staged SELL-32 one rules it out.
+  const bool onchip = A->fwd.sell_cols_global.ptr != nullptr &&
+                      (!A->kernel_set || A->kernel == SPMV_KERNEL_STAGED);
+  // The other fused kernels stream the staged product's tile table.
+  const bool staged = sp.kind == ProductKind::Staged && cg_tiles(A, sp).ok;
+  if (!onchip && !staged) return;
+  if (staged) {
+    const DevCsr::StagedTable& tiles = cg_tiles(A, sp);
+    w.tiles = tiles.desc.as<StagedDesc>();
+    w.ntiles = tiles.ntiles;
+    w.fused_args = k1_args(A, w, w.product);
+  }
   w.bar.reserve(sizeof(unsigned long long));
-  w.fused_args = k1_args(A, w, w.product);
 
   if (!mode.empty()) {
     FusedPlan p;
     bool fits = false;
-    if (mode == "1:smem") fits = plan_fused<CgFusedOne, true>(A, sp, p);
+    if (mode == "1:tmem:m") fits = onchip && plan_onchip(A, p);
+    else if (!staged) fits = false;
+    else if (mode == "1:smem") fits = plan_fused<CgFusedOne, true>(A, sp, p);
     else if (mode == "2:smem") fits = plan_fused<CgFusedTwo, true>(A, sp, p);
     else if (mode == "1:global") fits = plan_fused<CgFusedOne, false>(A, sp, p);
     else if (mode == "2:global") fits = plan_fused<CgFusedTwoDeep, false>(A, sp, p);
@@ -988,19 +1316,28 @@ void choose_form(spmv_matrix A, CgWorkspace& w) {
     else if (mode == "2:smem:m") fits = plan_fused<CgFusedTwo, true, true>(A, sp, p);
     else if (mode == "3:global:m") fits = plan_fused<CgFusedThree, false, true>(A, sp, p);
     require(fits, "spmv: SPMV_B200_CG_FUSED must be 0 or a fused plan that fits this matrix "
-                  "(1:smem, 2:smem, 1:global, 2:global, 3:global, 2:smem:m, 3:global:m)");
+                  "(1:smem, 2:smem, 1:global, 2:global, 3:global, 2:smem:m, 3:global:m, "
+                  "1:tmem:m)");
     use_plan(w, p);
     return;
   }
   std::vector<FusedPlan> plans;
   {
-    FusedPlan p1, p2, p3, p4, p5, p6;
-    if (plan_fused<CgFusedOne, true>(A, sp, p1)) plans.push_back(std::move(p1));
-    if (plan_fused<CgFusedTwo, true>(A, sp, p2)) plans.push_back(std::move(p2));
-    if (plan_fused<CgFusedTwoDeep, false>(A, sp, p3)) plans.push_back(std::move(p3));
-    if (plan_fused<CgFusedThree, false>(A, sp, p4)) plans.push_back(std::move(p4));
-    if (plan_fused<CgFusedTwo, true, true>(A, sp, p5)) plans.push_back(std::move(p5));
-    if (plan_fused<CgFusedThree, false, true>(A, sp, p6)) plans.push_back(std::move(p6));
+    FusedPlan p0, p1, p2, p3, p4, p5, p6;
+    const bool fits = onchip && plan_onchip(A, p0);
+    if (fits) plans.push_back(std::move(p0));
+    // Where the on-chip form fits, the others have not been faster (7-point
+    // 128^3: 40.0 us per iteration against 42.4 to 55.3; 96^3: 18.9 against
+    // 22.3 to 28.9; 5-point 1024^2: 15.6 against 20.3 to 24.3), so they are not
+    // timed.
+    if (staged && !fits) {
+      if (plan_fused<CgFusedOne, true>(A, sp, p1)) plans.push_back(std::move(p1));
+      if (plan_fused<CgFusedTwo, true>(A, sp, p2)) plans.push_back(std::move(p2));
+      if (plan_fused<CgFusedTwoDeep, false>(A, sp, p3)) plans.push_back(std::move(p3));
+      if (plan_fused<CgFusedThree, false>(A, sp, p4)) plans.push_back(std::move(p4));
+      if (plan_fused<CgFusedTwo, true, true>(A, sp, p5)) plans.push_back(std::move(p5));
+      if (plan_fused<CgFusedThree, false, true>(A, sp, p6)) plans.push_back(std::move(p6));
+    }
   }
   if (plans.empty()) return;
   cudaStream_t s = A->comm->stream;
@@ -1013,6 +1350,10 @@ void choose_form(spmv_matrix A, CgWorkspace& w) {
   for (size_t i = 0; i < plans.size(); ++i) {
     use_plan(w, plans[i]);
     const float t = time_iterations(w, s, its);
+    debug_log("cg form " + std::to_string(plans[i].cps) +
+              (plans[i].tmem ? ":tmem" : plans[i].rs ? ":smem" : ":global") +
+              (plans[i].merged ? ":m " : " ") + std::to_string(t * 1e3f / its) +
+              " us per iteration");
     if (!w.fused) continue;  // the plan's launch was refused (graph form ran)
     if (t < best) {
       best = t;
@@ -1065,6 +1406,16 @@ bool fused_plan(spmv_matrix A, const DevCsr::StagedTable& t, const void* fn, int
   std::vector<FusedCta> ctas;
   const int64_t longest = fused_ctas(A, t, grid, ctas);
   const int64_t smem = stage_smem + (longest * rs_bytes + 15) / 16 * 16;
+  if (!fused_fits(comm, fn, block, cps, smem, plan)) return false;
+  plan.grid = grid;
+  plan.cps = cps;
+  plan.rs = rs_bytes > 0;
+  plan.ctas = std::move(ctas);
+  return true;
+}
+
+bool fused_fits(spmv_comm comm, const void* fn, int block, int cps, int64_t smem,
+                FusedPlan& plan) {
   int optin = 0;
   SPMVB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin,
                                     comm->device));
@@ -1074,14 +1425,15 @@ bool fused_plan(spmv_matrix A, const DevCsr::StagedTable& t, const void* fn, int
   SPMVB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   int nb = 0;
   SPMVB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, block, size_t(smem)));
-  if (nb < cps) return false;
+  if (nb < cps) {
+    debug_log("fused plan: " + std::to_string(nb) + " of " + std::to_string(cps) +
+              " CTAs fit, registers " + std::to_string(fa.numRegs) + ", shared memory " +
+              std::to_string(smem) + " + " + std::to_string(fa.sharedSizeBytes));
+    return false;
+  }
   plan.fn = fn;
-  plan.grid = grid;
   plan.block = block;
   plan.smem = int(smem);
-  plan.cps = cps;
-  plan.rs = rs_bytes > 0;
-  plan.ctas = std::move(ctas);
   return true;
 }
 
@@ -1166,6 +1518,7 @@ CgForm cg_form(spmv_matrix A) {
   f.cps = w.fused ? w.fused_cps : 0;
   f.rs = w.fused && w.fused_rs;
   f.merged = w.fused && w.fused_mg;
+  f.tmem = w.fused && w.fused_tm;
   return f;
 }
 

@@ -228,6 +228,16 @@ struct DevPart {
   int64_t snnz = 0;     // SELL entries including padding
 };
 
+// Items of consecutive SELL slices of a rank, all ranks in order (their format
+// is in sell_ring.cuh); on the host the items' first global rows and, at
+// [nitems], the row count.
+struct ItemTable {
+  bool built = false, ok = false;
+  int nitems = 0;
+  DevBuf desc;
+  std::vector<int32_t> row;
+};
+
 // A device CSR (all ranks concatenated) plus the derived column arrays.
 struct DevCsr {
   std::vector<DevPart> parts;
@@ -264,6 +274,7 @@ struct DevCsr {
     };
     std::vector<Rows> rows;
   } staged[4];
+  ItemTable items[2];  // of one and of two slices
   // Row statistics (over all ranks).
   double mean_row = 0;
   int64_t max_row = 0;
@@ -405,12 +416,23 @@ struct FusedCta {
 // each; returns the longest run's row count.
 int64_t fused_ctas(spmv_matrix A, const DevCsr::StagedTable& t, int grid,
                    std::vector<FusedCta>& out);
+// Launch shape of spmv_cg's on-chip form (cg.cu cg_onchip).
+struct OnchipShape {
+  const double* vals = nullptr;   // SELL values and indices of all ranks
+  const void* idx = nullptr;
+  const int4* items = nullptr;    // item table (sell_ring.cuh)
+  int per_warp = 0;               // items per warp at most
+  int cols = 0;                   // tensor memory columns per slice: r, y (4) and x (6)
+  int alloc = 0;                  // columns allocated per CTA
+};
 struct FusedPlan {
   const void* fn = nullptr;
   int grid = 0, block = 0, smem = 0;
   int cps = 0;      // CTAs per SM
   bool rs = false;  // a vector of the CTA's rows kept in shared memory
   bool merged = false;  // spmv_cg's merged-update form (two grid syncs per iteration)
+  bool tmem = false;    // its on-chip form
+  OnchipShape onchip;
   std::vector<FusedCta> ctas;
 };
 // A plan for kernel `fn` of `block` threads at `cps` CTAs per SM over the
@@ -418,6 +440,14 @@ struct FusedPlan {
 // of the longest run in shared memory; false when it does not fit.
 bool fused_plan(spmv_matrix A, const DevCsr::StagedTable& t, const void* fn, int block,
                 int cps, int64_t stage_smem, int rs_bytes, FusedPlan& plan);
+// Whether `cps` CTAs of `block` threads of `fn` with `smem` bytes of dynamic
+// shared memory fit an SM; sets the plan's kernel, block and shared memory.
+bool fused_fits(spmv_comm comm, const void* fn, int block, int cps, int64_t smem,
+                FusedPlan& plan);
+// The table of items of 1 or 2 slices of the forward SELL layout over the
+// global rows (built once); ok is false when the layout does not fit its fields
+// (for 2: a slice of more than 255 columns).
+const ItemTable& item_table(spmv_matrix A, int slices);
 // Bound of each grid wait of a fused solve: 2 s, or SPMV_B200_WAIT_LIMIT_NS.
 unsigned long long fused_wait_ns();
 // The products chosen by the built solver workspaces (fails if none).
@@ -428,6 +458,7 @@ struct CgForm {
   int cps = 0;
   bool rs = false;
   bool merged = false;  // two grid syncs per iteration (spmv_cg's fused form only)
+  bool tmem = false;    // r (and y) in tensor memory
 };
 CgForm cg_form(spmv_matrix A);
 CgForm ir_form(spmv_matrix A);  // spmv_cg_mixed's

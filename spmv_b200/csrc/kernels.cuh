@@ -464,4 +464,108 @@ __device__ __forceinline__ bool coop_grid_sum_n(const double (&v)[N], double* pa
   return true;
 }
 
+// Warp sums of N values at once; value j's total is in the lanes for which
+// warp_total_of(lane) == j (every lane for N = 1).  Four values are folded onto
+// quarters of the warp first: 6 exchanges instead of 20.
+template <int N>
+__device__ __forceinline__ double warp_totals(const double (&v)[N]) {
+  const int lane = int(threadIdx.x) & 31;
+  double x;
+  if constexpr (N == 4) {
+    const bool hi = (lane & 16) != 0, mid = (lane & 8) != 0;
+    double a = hi ? v[2] : v[0], b = hi ? v[3] : v[1];
+    a += __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], 16);
+    b += __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], 16);
+    x = mid ? b : a;
+    x += __shfl_xor_sync(0xffffffffu, mid ? a : b, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  } else {
+    x = 0.0;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      double t = v[j];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (N == 1 || lane == j) x = t;
+    }
+  }
+  return x;
+}
+// The value whose total warp_totals leaves in this lane, if it is the lane
+// that reports it (-1 otherwise).
+template <int N>
+__device__ __forceinline__ int warp_total_of() {
+  const int lane = int(threadIdx.x) & 31;
+  if (N == 4) return (lane & 7) == 0 ? lane >> 3 : -1;
+  return lane < N ? lane : -1;
+}
+
+// N sums at once: parts holds N partials per CTA (CTA b's at parts[N b .. N b
+// + N - 1]); every thread of every CTA gets the same N totals, in a fixed order
+// (lanes, warps, then CTAs by lane, lanes, warps).  No
+// step is serial over warps or CTAs, as coop_grid_sum_n's are: a sum of four at
+// 148 CTAs of 24 warps took 4.1 us that way, of which 1.5 are the barrier, and
+// takes 2.9 this way.  (With 12 warps and 296 or 444 CTAs the serial steps are
+// short and this form's registers cost more than it gains: the fused mixed
+// solve runs 43.9 and 47.9 us per iteration with it against 42.9 and 41.0.
+// Slots of 16 bytes, value and tag, that every CTA polls instead of a counter
+// were slower still: 5.5 us for the sum and 5 for the barrier.)
+template <int NT, int N>
+struct GridTotals {
+  static constexpr int PV = NT / 32 / N;  // warps per value when the CTAs' partials are added
+  double red[N][NT / 32];
+  double part[N][PV];
+  int ok;
+};
+
+template <int NT, int N>
+__device__ __forceinline__ bool coop_grid_totals(const double (&v)[N], double* parts,
+                                                unsigned long long* count,
+                                                unsigned long long target, int* err,
+                                                unsigned long long limit_ns, GridTotals<NT, N>& s,
+                                                double (&total)[N]) {
+  constexpr int NW = NT / 32;
+  static_assert(NW <= 32, "one lane per warp");
+  const int warp = int(threadIdx.x) >> 5, lane = int(threadIdx.x) & 31;
+  const int mine = warp_total_of<N>();
+  {
+    const double x = warp_totals<N>(v);
+    if (mine >= 0) s.red[mine][warp] = x;
+  }
+  named_sync(1, NT);
+  if (warp == 0) {
+    double w[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) w[j] = lane < NW ? s.red[j][lane] : 0.0;
+    const double x = warp_totals<N>(w);
+    if (mine >= 0) __stcg(parts + N * blockIdx.x + mine, x);
+    __syncwarp();
+    if (lane == 0) s.ok = grid_arrive_wait(count, target, err, limit_ns);
+  }
+  named_sync(1, NT);
+  if (!s.ok) return false;
+  // PV warps per value: each sums the partials of its lanes' CTAs.
+  constexpr int PV = GridTotals<NT, N>::PV;
+  const int j = warp / PV, q = warp % PV;
+  if (j < N) {
+    double x = 0.0;
+#pragma unroll 2
+    for (unsigned int b = 32u * unsigned(q) + unsigned(lane); b < gridDim.x; b += 32u * PV)
+      x += __ldcg(parts + N * b + j);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if (lane == 0) s.part[j][q] = x;
+  }
+  named_sync(1, NT);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int r = 0; r < PV; ++r) t[r % 4] += s.part[i][r];
+    total[i] = (t[0] + t[1]) + (t[2] + t[3]);
+  }
+  return true;
+}
+
 }  // namespace spmvb

@@ -187,6 +187,50 @@ const DevCsr::StagedTable& staged_table(DevCsr& C, int entry_bytes, int max_entr
   return t;
 }
 
+const ItemTable& item_table(spmv_matrix A, int slices) {
+  DevCsr& C = A->fwd;
+  require(slices == 1 || slices == 2, "spmv: items have one or two slices");
+  ItemTable& t = C.items[slices - 1];
+  if (t.built) return t;
+  require(C.sell_built, "spmv: the item table needs the SELL layout");
+  std::vector<int4> desc;
+  std::vector<int32_t> row;
+  bool ok = true;
+  int64_t row0 = 0;
+  for (const DevPart& D : C.parts) {
+    const int32_t* so = C.h_sell_off.data() + D.sl_off;
+    const int nslices = (D.nrows + 31) / 32;
+    auto cols = [&](int s) { return s < nslices ? (so[s + 1] - so[s]) / 32 : 0; };
+    auto rows = [&](int s) { return s < nslices ? std::min(32, D.nrows - s * 32) : 0; };
+    for (int s = 0; s < nslices; s += slices) {
+      const int64_t first = (D.sz_off + so[s]) / 32, g = row0 + int64_t(s) * 32;
+      ok = ok && first < (int64_t(1) << 31) && g < (int64_t(1) << 31) - 64;
+      uint32_t z;
+      if (slices == 1) {
+        ok = ok && cols(s) < (1 << 24);
+        z = uint32_t(cols(s)) | uint32_t(rows(s)) << 24;
+      } else {
+        ok = ok && cols(s) < 256 && cols(s + 1) < 256;
+        z = uint32_t(cols(s)) | uint32_t(cols(s + 1)) << 8 | uint32_t(rows(s)) << 16 |
+            uint32_t(rows(s + 1)) << 24;
+      }
+      desc.push_back(make_int4(int(first), int(g), int(z), 0));
+      row.push_back(int32_t(g));
+    }
+    row0 += D.nrows;
+  }
+  t.built = true;
+  t.ok = ok && !desc.empty();
+  if (!t.ok) return t;
+  t.nitems = int(desc.size());
+  row.push_back(int32_t(row0));
+  t.row = std::move(row);
+  t.desc.reserve(sizeof(int4) * desc.size());
+  SPMVB_CUDA(cudaMemcpy(t.desc.ptr, desc.data(), sizeof(int4) * desc.size(),
+                        cudaMemcpyHostToDevice));
+  return t;
+}
+
 void refresh_sell_values(spmv_matrix A) {
   DevCsr& C = A->fwd;
   if (!C.sell_built) return;
