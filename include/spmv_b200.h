@@ -110,6 +110,16 @@ int spmv_comm_destroy(spmv_comm comm);
 int spmv_comm_size(spmv_comm comm, int* size);
 int spmv_comm_device(spmv_comm comm, int* device);
 int spmv_comm_stream(spmv_comm comm, void** stream);
+/* Orders the communicator's stream against the caller's `stream` with
+ * device-side events (the host does not wait): leave = 0 before a call on
+ * device vectors that work on `stream` produced, leave = 1 after it, before
+ * work on `stream` uses the results.  Nothing to do when they are one stream.
+ * leave = 2 and 3: the same around calls that only put work on a stream
+ * (update, reverse_update, mult, transpmult, mult_block, sample_outer); when
+ * `stream` is the legacy default stream (NULL) and the communicator made its
+ * own stream, which spmv_comm_stream has not handed out, the calls this thread
+ * makes in between put their work on `stream` itself. */
+int spmv_comm_fence(spmv_comm comm, void* stream, int leave);
 int spmv_comm_synchronize(spmv_comm comm);
 
 /* ------------------------------------------------------------------------ */

@@ -81,6 +81,7 @@ _SIGS = {
     "spmv_comm_size": [_p, C.POINTER(_int)],
     "spmv_comm_device": [_p, C.POINTER(_int)],
     "spmv_comm_stream": [_p, C.POINTER(_p)],
+    "spmv_comm_fence": [_p, _p, _int],
     "spmv_comm_synchronize": [_p],
     "spmv_l2gmap_create": [_p, C.POINTER(_i64), C.POINTER(C.POINTER(_i64)),
                            C.POINTER(_i64), C.POINTER(_p)],
@@ -175,15 +176,21 @@ def check(status: int) -> None:
 
 
 def call(name: str, *args) -> None:
-    check(getattr(lib(), name)(*args))
+    status = getattr(_lib or lib(), name)(*args)
+    if status != SUCCESS:
+        check(status)
+
+
+_PTR_ARRAYS: dict = {}
 
 
 def ptr_array(ptrs) -> "C.Array":
     """void*[n] from a sequence of integer addresses (or None)."""
-    arr = (C.c_void_p * max(1, len(ptrs)))()
-    for i, p in enumerate(ptrs):
-        arr[i] = p
-    return arr
+    n = len(ptrs)
+    t = _PTR_ARRAYS.get(n)
+    if t is None:
+        t = _PTR_ARRAYS[n] = C.c_void_p * max(1, n)
+    return t(*ptrs)
 
 
 def declared_symbols(header: Path | None = None):

@@ -25,8 +25,28 @@ _DTYPES = {np.dtype(np.float64): _lib.FLOAT64, np.dtype(np.float32): _lib.FLOAT3
 _NP_OF = {v: k for k, v in _DTYPES.items()}
 
 
+_TORCH_TYPES: dict = {}
+
+
 def _is_torch(v) -> bool:
-    return type(v).__module__.startswith("torch")
+    t = type(v)
+    r = _TORCH_TYPES.get(t)
+    if r is None:
+        r = _TORCH_TYPES[t] = t.__module__.startswith("torch")
+    return r
+
+
+_raw_stream = None
+
+
+def _user_stream(device: int) -> int:
+    """torch's current stream on `device` as a cudaStream_t handle."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+            lambda d: torch.cuda.current_stream(d).cuda_stream)
+    return _raw_stream(device)
 
 
 class _Fence:
@@ -38,54 +58,70 @@ class _Fence:
     work (that produces the outputs).  Both waits are device-side events; the
     host does not block."""
 
-    def __init__(self, comm, device: bool):
+    __slots__ = ("comm", "stream", "mode")
+
+    def __init__(self, comm, device: bool, mode: int = 0):
+        # mode 2: the calls inside only put work on a stream, and may put it on
+        # torch's (spmv_comm_fence).
         self.comm = comm if device else None
+        self.mode = mode
 
     def __enter__(self):
         if self.comm is not None:
-            import torch
-            self.torch_stream = torch.cuda.current_stream(self.comm.device)
-            self.lib_stream = self.comm.torch_stream()
-            self.lib_stream.wait_stream(self.torch_stream)
+            # The events are the library's (two per thread): an event made and
+            # two torch stream objects per wait cost 10 us of a small call.
+            self.stream = _user_stream(self.comm.device)
+            call("spmv_comm_fence", self.comm._h, self.stream, self.mode)
         return self
 
     def __exit__(self, *exc):
         if self.comm is not None:
-            self.torch_stream.wait_stream(self.lib_stream)
+            call("spmv_comm_fence", self.comm._h, self.stream, self.mode + 1)
         return False
+
+
+_TORCH_DTYPES = None
+
+
+def _torch_dtypes():
+    global _TORCH_DTYPES
+    if _TORCH_DTYPES is None:
+        import torch
+        _TORCH_DTYPES = {torch.float64: _lib.FLOAT64, torch.float32: _lib.FLOAT32,
+                         torch.complex64: _lib.COMPLEX64, torch.complex128: _lib.COMPLEX128}
+    return _TORCH_DTYPES
 
 
 def _vec_info(vecs: Sequence):
     """(memory kind, dtype code, addresses) of a per-rank vector list."""
     if len(vecs) == 0:
         raise SpmvError(_lib.ERROR_INVALID_ARGUMENT, "spmv: empty vector list")
-    kinds = {_is_torch(v) for v in vecs}
-    if len(kinds) != 1:
-        raise SpmvError(_lib.ERROR_INVALID_ARGUMENT,
-                        "spmv: mix of host and device vectors")
-    if kinds.pop():
-        import torch
+    on_device = _is_torch(vecs[0])
+    for v in vecs:
+        if _is_torch(v) != on_device:
+            raise SpmvError(_lib.ERROR_INVALID_ARGUMENT,
+                            "spmv: mix of host and device vectors")
+    dtype, one_dtype, ptrs = vecs[0].dtype if hasattr(vecs[0], "dtype") else None, True, []
+    if on_device:
         for v in vecs:
             if not v.is_cuda or not v.is_contiguous():
                 raise SpmvError(_lib.ERROR_INVALID_ARGUMENT,
                                 "spmv: device vectors must be contiguous CUDA tensors")
-        tdt = {torch.float64: _lib.FLOAT64, torch.float32: _lib.FLOAT32,
-               torch.complex64: _lib.COMPLEX64, torch.complex128: _lib.COMPLEX128}
-        dts = {tdt.get(v.dtype, -1) for v in vecs}
-        ptrs = [v.data_ptr() for v in vecs]
-        mem = _lib.MEMORY_DEVICE
+            one_dtype = one_dtype and v.dtype == dtype
+            ptrs.append(v.data_ptr())
+        code, mem = _torch_dtypes().get(dtype), _lib.MEMORY_DEVICE
     else:
         for v in vecs:
             if not (isinstance(v, np.ndarray) and v.flags.c_contiguous):
                 raise SpmvError(_lib.ERROR_INVALID_ARGUMENT,
                                 "spmv: host vectors must be contiguous numpy arrays")
-        dts = {_DTYPES.get(v.dtype, -1) for v in vecs}
-        ptrs = [v.ctypes.data for v in vecs]
-        mem = _lib.MEMORY_HOST
-    if len(dts) != 1 or -1 in dts:
+            one_dtype = one_dtype and v.dtype == dtype
+            ptrs.append(v.ctypes.data)
+        code, mem = _DTYPES.get(dtype), _lib.MEMORY_HOST
+    if not one_dtype or code is None:
         raise SpmvError(_lib.ERROR_INVALID_ARGUMENT,
                         "spmv: vectors need one supported dtype")
-    return mem, dts.pop(), ptrs
+    return mem, code, ptrs
 
 
 class Comm:
@@ -121,8 +157,8 @@ class Comm:
                                                  device=torch.device("cuda", self.device))
         return self._ts
 
-    def fence(self, vecs) -> "_Fence":
-        return _Fence(self, bool(vecs) and _is_torch(vecs[0]))
+    def fence(self, vecs, mode: int = 0) -> "_Fence":
+        return _Fence(self, bool(vecs) and _is_torch(vecs[0]), mode)
 
     def close(self) -> None:
         if getattr(self, "_h", None) and self._h.value:
@@ -206,13 +242,13 @@ class L2GMap:
     def update(self, vecs: Sequence) -> None:
         """L2GMap::update (L2GMap.cpp:126-150) on all ranks' vectors, in place."""
         mem, dt, ptrs = _vec_info(vecs)
-        with self.comm.fence(vecs):
+        with self.comm.fence(vecs, 2):
             call("spmv_l2gmap_update", self._h, dt, mem, ptr_array(ptrs))
 
     def reverse_update(self, vecs: Sequence) -> None:
         """L2GMap::reverse_update (L2GMap.cpp:152-170), in place."""
         mem, dt, ptrs = _vec_info(vecs)
-        with self.comm.fence(vecs):
+        with self.comm.fence(vecs, 2):
             call("spmv_l2gmap_reverse_update", self._h, dt, mem, ptr_array(ptrs))
 
     def close(self) -> None:
@@ -320,7 +356,7 @@ class Matrix:
             else:
                 out = [np.empty((n, k), dtype=X[0].dtype) for n in self.nrows]
         _, _, optrs = _vec_info(out)
-        with self.comm.fence(X):
+        with self.comm.fence(X, 2):
             call("spmv_matrix_mult_block", self._h, k, mem, ptr_array(ptrs),
                  ptr_array(optrs))
         return out
@@ -366,8 +402,8 @@ class Matrix:
 
     def _alloc_like(self, x0, lens):
         if _is_torch(x0):
-            import torch
-            return [torch.empty(n, dtype=x0.dtype, device=x0.device) for n in lens]
+            new = x0.detach().new_empty
+            return [new(n) for n in lens]
         return [np.empty(n, dtype=x0.dtype) for n in lens]
 
     def mult(self, x: Sequence, out: Optional[List] = None) -> List:
@@ -375,7 +411,7 @@ class Matrix:
         mem, dt, ptrs = _vec_info(x)
         y = out if out is not None else self._alloc_like(x[0], self.nrows)
         _, _, yptrs = _vec_info(y)
-        with self.comm.fence(x):
+        with self.comm.fence(x, 2):
             call("spmv_matrix_mult", self._h, mem, ptr_array(ptrs), ptr_array(yptrs))
         return y
 
@@ -386,7 +422,7 @@ class Matrix:
         mem, dt, ptrs = _vec_info(x)
         y = out if out is not None else self._alloc_like(x[0], self.ncols)
         _, _, yptrs = _vec_info(y)
-        with self.comm.fence(x):
+        with self.comm.fence(x, 2):
             call("spmv_matrix_transpmult", self._h, mem, ptr_array(ptrs),
                  ptr_array(yptrs))
         return y
@@ -400,7 +436,7 @@ class Matrix:
         if out is None:
             out = self._alloc_like(lam[0], [self.nnz(r) for r in range(self.comm.size)])
         _, _, optrs = _vec_info(out)
-        with self.comm.fence(lam):
+        with self.comm.fence(lam, 2):
             call("spmv_matrix_sample_outer", self._h, mem, float(scale),
                  ptr_array(lptrs), ptr_array(xptrs), ptr_array(optrs))
         return out

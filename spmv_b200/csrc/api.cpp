@@ -46,6 +46,75 @@ DeviceGuard::~DeviceGuard() {
 
 namespace {
 
+// One event per thread and device, made on first use: it is recorded and the
+// other stream made to wait for it at once, so a thread can use its own again
+// for the next pair.
+struct FenceEvents {
+  std::vector<cudaEvent_t> ev;  // per device
+  cudaEvent_t get(int device) {
+    if (int(ev.size()) <= device) ev.resize(size_t(device) + 1, nullptr);
+    if (!ev[size_t(device)])
+      SPMVB_CUDA(cudaEventCreateWithFlags(&ev[size_t(device)], cudaEventDisableTiming));
+    return ev[size_t(device)];
+  }
+  ~FenceEvents() {
+    for (cudaEvent_t e : ev)
+      if (e) soft_check(cudaEventDestroy(e), "cudaEventDestroy");
+  }
+};
+thread_local FenceEvents g_fence;
+// The communicator's stream whose direct fence this thread is in.
+thread_local const WorkStream* g_direct = nullptr;
+
+// Work put on `after` from here on waits for the work now on `before`.
+void order_streams(int device, cudaStream_t before, cudaStream_t after) {
+  cudaEvent_t e = g_fence.get(device);
+  SPMVB_CUDA(cudaEventRecord(e, before));
+  SPMVB_CUDA(cudaStreamWaitEvent(after, e, 0));
+}
+
+}  // namespace
+
+cudaStream_t WorkStream::get() const {
+  const std::lock_guard<std::mutex> lock(mu_);
+  if (g_direct == this) {
+    if (own_ahead_) {  // another thread's work since the fence began
+      order_streams(device_, own_, nullptr);
+      own_ahead_ = false;
+    }
+    default_ahead_ = true;
+    return nullptr;
+  }
+  if (default_ahead_) {
+    order_streams(device_, nullptr, own_);
+    default_ahead_ = false;
+  }
+  own_ahead_ = true;
+  return own_;
+}
+
+void WorkStream::hand_out() const {
+  (void)get();  // what follows on the handle is behind the direct work
+  const std::lock_guard<std::mutex> lock(mu_);
+  given_ = true;
+}
+
+bool WorkStream::begin_direct(int device) const {
+  const std::lock_guard<std::mutex> lock(mu_);
+  if (given_ || g_direct != nullptr) return false;
+  device_ = device;
+  g_direct = this;
+  return true;
+}
+
+bool WorkStream::end_direct() const {
+  if (g_direct != this) return false;
+  g_direct = nullptr;
+  return true;
+}
+
+namespace {
+
 void check_comm(spmv_comm c) { require(c != nullptr, "spmv: communicator is NULL"); }
 void check_map(spmv_l2gmap m) { require(m != nullptr, "spmv: L2GMap is NULL"); }
 void check_mat(spmv_matrix A) { require(A != nullptr, "spmv: Matrix is NULL"); }
@@ -119,6 +188,20 @@ void upload_csr(spmv_matrix A) {
   }
 }
 
+// The host copy of the values, read back if the device's are newer.
+void fresh_host_values(spmv_matrix A) {
+  if (!A->h_vals_stale) return;
+  DeviceGuard dg(A->comm->device);
+  const size_t es = dtype_size(A->dtype);
+  for (int r = 0; r < A->comm->size; ++r) {
+    const DevPart& D = A->fwd.parts[r];
+    if (D.nnz > 0)
+      SPMVB_CUDA(cudaMemcpy(A->h_vals[r].data(), A->fwd.vals.as<char>() + D.nz_off * es,
+                            es * D.nnz, cudaMemcpyDeviceToHost));
+  }
+  A->h_vals_stale = false;
+}
+
 // Global column numbering for the fused-halo layout: an owned column c of
 // rank r is col_range[r] + c, a ghost column is its global index.
 void build_global_cols(spmv_matrix A) {
@@ -172,6 +255,7 @@ void build_global_cols(spmv_matrix A) {
 // (Matrix.cpp:206-211) accumulates them.
 void build_transpose(spmv_matrix A) {
   if (A->trn_built) return;
+  fresh_host_values(A);
   DevCsr& T = A->trn;
   const int P = A->comm->size;
   const size_t es = dtype_size(A->dtype);
@@ -241,7 +325,7 @@ void release_comm(spmv_comm comm) {
   if (comm->device >= 0) {
     DeviceGuard dg(comm->device);
     if (comm->own_stream)
-      soft_check(cudaStreamDestroy(comm->stream), "cudaStreamDestroy");
+      soft_check(cudaStreamDestroy(comm->stream.own()), "cudaStreamDestroy");
     comm->stage_in.release();
     comm->stage_out.release();
   }
@@ -472,9 +556,11 @@ int spmv_comm_create(int device, void* stream, int size, spmv_comm* out) {
       DeviceGuard dg(device);
       SPMVB_CUDA(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device));
       if (stream) {
-        c->stream = static_cast<cudaStream_t>(stream);
+        c->stream.set(static_cast<cudaStream_t>(stream));
       } else {
-        SPMVB_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+        cudaStream_t made = nullptr;
+        SPMVB_CUDA(cudaStreamCreateWithFlags(&made, cudaStreamNonBlocking));
+        c->stream.set(made);
         c->own_stream = true;
       }
     }
@@ -508,7 +594,33 @@ int spmv_comm_stream(spmv_comm comm, void** stream) {
   return guard([&] {
     check_comm(comm);
     require(stream, "spmv: NULL output");
-    *stream = comm->stream;
+    *stream = comm->stream.own();
+    if (comm->device >= 0 && comm->own_stream) {
+      DeviceGuard dg(comm->device);
+      comm->stream.hand_out();
+    }
+  });
+}
+
+int spmv_comm_fence(spmv_comm comm, void* stream, int leave) {
+  return guard([&] {
+    check_comm(comm);
+    comm->require_device();
+    require(leave >= 0 && leave <= 3, "spmv: leave must be 0, 1, 2 or 3");
+    cudaStream_t user = static_cast<cudaStream_t>(stream);
+    if (user == comm->stream.own()) return;
+    if (leave >= 2 && user == nullptr && comm->own_stream) {
+      if (leave == 3 && comm->stream.end_direct()) return;
+      if (leave == 2) {
+        DeviceGuard dg(comm->device);
+        if (comm->stream.begin_direct(comm->device)) return;
+      }
+    }
+    DeviceGuard dg(comm->device);
+    if (leave & 1)
+      order_streams(comm->device, comm->stream, user);
+    else
+      order_streams(comm->device, user, comm->stream);
   });
 }
 
@@ -781,6 +893,7 @@ int spmv_matrix_csr(spmv_matrix A, int rank, const int32_t** rowptr,
     require(rowptr && colind && values, "spmv: NULL output");
     *rowptr = A->h_rowptr[rank].data();
     *colind = A->h_colind[rank].data();
+    fresh_host_values(A);
     *values = A->h_vals[rank].data();
   });
 }
@@ -809,21 +922,32 @@ int spmv_matrix_set_values(spmv_matrix A, spmv_memory memory,
     const int P = A->comm->size;
     const size_t es = dtype_size(A->dtype);
     DeviceGuard dg(A->comm->device);
-    for (int r = 0; r < P; ++r) {
-      const int64_t nnz = A->h_rowptr[r][A->nrows[r]];
-      if (nnz == 0) continue;
-      require(values[r] != nullptr, "spmv: NULL value array");
-      if (memory == SPMV_MEMORY_HOST) {
+    for (int r = 0; r < P; ++r)
+      require(A->h_rowptr[r][A->nrows[r]] == 0 || values[r] != nullptr, "spmv: NULL value array");
+    if (memory == SPMV_MEMORY_HOST) {
+      for (int r = 0; r < P; ++r) {
+        const int64_t nnz = A->h_rowptr[r][A->nrows[r]];
+        if (nnz == 0) continue;
         const unsigned char* vb = static_cast<const unsigned char*>(values[r]);
         std::memcpy(A->h_vals[r].data(), vb, nnz * es);
-      } else {
-        A->comm->require_device();
-        SPMVB_CUDA(cudaMemcpy(A->h_vals[r].data(), values[r], nnz * es,
-                              cudaMemcpyDeviceToHost));
+        if (A->comm->device >= 0)
+          SPMVB_CUDA(cudaMemcpy(A->fwd.vals.as<char>() + A->fwd.parts[r].nz_off * es,
+                                A->h_vals[r].data(), nnz * es, cudaMemcpyHostToDevice));
       }
-      if (A->comm->device >= 0)
-        SPMVB_CUDA(cudaMemcpy(A->fwd.vals.as<char>() + A->fwd.parts[r].nz_off * es,
-                              A->h_vals[r].data(), nnz * es, cudaMemcpyHostToDevice));
+      A->h_vals_stale = false;
+    } else {
+      // The device copy only: the host copy is read back when something asks
+      // for it (5.2 M FP64 values: 5 ms for both copies through the host).
+      A->comm->require_device();
+      cudaStream_t s = A->comm->stream;
+      A->h_vals_stale = true;
+      for (int r = 0; r < P; ++r) {
+        const int64_t nnz = A->h_rowptr[r][A->nrows[r]];
+        if (nnz > 0)
+          SPMVB_CUDA(cudaMemcpyAsync(A->fwd.vals.as<char>() + A->fwd.parts[r].nz_off * es,
+                                     values[r], nnz * es, cudaMemcpyDeviceToDevice, s));
+      }
+      SPMVB_CUDA(cudaStreamSynchronize(s));
     }
     // Derived copies are rebuilt on next use (the mixed solver's graph holds
     // the FP32 copy's address, so it goes too).
