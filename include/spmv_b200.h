@@ -401,8 +401,8 @@ typedef enum spmv_batch_precision {
                             FP64 residual                                       */
 } spmv_batch_precision;
 
-/* Launch shape of the batched kernel (0 in a field of spmv_batch_set_config:
- * keep the current value). */
+/* Launch shape of the lockstep batched kernel (0 in a field of
+ * spmv_batch_set_config: keep the current value). */
 typedef struct spmv_batch_config {
   int ctas_per_sm;   /* CTAs of 512 threads per SM: 1 or 2                     */
   int tile_rows;     /* rows a warp takes at a time: 128, 256 or 512           */
@@ -432,7 +432,12 @@ int spmv_batch_destroy(spmv_batch batch);
  * spmv_batch_solve_ex, solved in the same launch with one product per
  * iteration for all its columns (its matrix read once per iteration). */
 int spmv_batch_set_block(spmv_batch batch, int system, int nrhs);
-/* Launch shape of the solves of one precision; see spmv_batch_config.
+/* A solve runs every system (and block column) in its own group of CTAs, its
+ * vectors on chip, when there are no more of them than SMs and their rows fit
+ * there (about 3 million in mixed precision, 1.2 in FP64); larger batches, and
+ * those whose launch shape spmv_batch_set_config has set, run in the lockstep
+ * kernel.  Launch shape of the lockstep solves of one precision; see
+ * spmv_batch_config.
  * spmv_batch_autotune times the candidates (ctas_per_sm x tile_rows x
  * rhs_lanes) on short solves of this batch in that precision and keeps the
  * fastest; with SPMV_B200_TUNE_CACHE naming a file the choice is cached by

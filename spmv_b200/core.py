@@ -556,6 +556,8 @@ class Batch:
 
     def set_config(self, ctas_per_sm: int = 0, tile_rows: int = 0, rhs_lanes: int = 0,
                    window: Optional[bool] = None, precision: str = "mixed") -> None:
+        """Launch shape of the lockstep kernel; solves of this precision then
+        use that kernel also where the batch would fit on chip."""
         w = 0 if window is None else (2 if window else 1)
         c = _lib.BatchConfig(int(ctas_per_sm), int(tile_rows), int(rhs_lanes), w, 0.0, 0)
         call("spmv_batch_set_config", self._h, self._PREC[precision], C.byref(c))
@@ -572,8 +574,8 @@ class Batch:
         return self._cfg(c)
 
     def autotune(self, precision: str = "mixed") -> dict:
-        """Times the launch shapes on short solves of this precision and keeps
-        the fastest for it."""
+        """Times the lockstep kernel's launch shapes on short solves of this
+        precision and keeps the fastest for it."""
         c = _lib.BatchConfig()
         call("spmv_batch_autotune", self._h, self._PREC[precision], C.byref(c))
         return self._cfg(c)

@@ -39,6 +39,15 @@ struct spmv_batch_s {
   spmvb::DevBuf stage;            // host-memory solves: b and x staged here
   spmvb::DevBuf prof;             // phase timeline (SPMV_B200_BATCH_PROFILE)
   std::vector<int64_t> part_off;  // per unit
+  // The on-chip form: slice table, plans (precision, with the block or not) and
+  // their device state.
+  spmvb::DevBuf oc_items;
+  struct Onchip {
+    bool planned = false;
+    spmvb::bat::OnchipPlan plan;
+    spmvb::DevBuf ctas;
+  } oc[2][2];
+  spmvb::DevBuf oc_p, oc_x, oc_b, oc_parts, oc_bars;
 };
 
 namespace spmvb {
@@ -58,6 +67,10 @@ constexpr int kProfCap = 1 << 16;
 // fallen 100x below its largest value since the last refinement (the
 // reliable-update criterion with delta = 0.01; squared norms compared).
 constexpr double kDelta2 = 1e-4;
+double delta2_of(const spmv_batch_s* B, spmv_batch_precision prec) {
+  if (prec != SPMV_BATCH_MIXED) return 0.0;
+  return B->plan.fits16 ? kDelta2 : 0.01;
+}
 // Rows of p the product phase stages per CTA (64 KB in FP32, kept as a ring
 // across a pass's chunks; 88 KB in FP64: two CTAs per SM still fit).
 constexpr int kWinRows32 = 16384;
@@ -274,21 +287,78 @@ bool run(spmv_batch B, spmv_batch_precision prec, const SolveIo& io, int kmax, d
   if (prec == SPMV_BATCH_MIXED) {
     if (d16) {
       Args<float, int16_t> a;
-      fill_args(B, a, io, kmax, rtol, kDelta2, cfg, dry);
+      fill_args(B, a, io, kmax, rtol, delta2_of(B, prec), cfg, dry);
       return launch_f32(&a, true, cfg, comm->num_sms, s, dry);
     }
     Args<float, int32_t> a;
-    fill_args(B, a, io, kmax, rtol, 0.01, cfg, dry);
+    fill_args(B, a, io, kmax, rtol, delta2_of(B, prec), cfg, dry);
     return launch_f32(&a, false, cfg, comm->num_sms, s, dry);
   }
   if (d16) {
     Args<double, int16_t> a;
-    fill_args(B, a, io, kmax, rtol, 0.0, cfg, dry);
+    fill_args(B, a, io, kmax, rtol, delta2_of(B, prec), cfg, dry);
     return launch_f64(&a, true, cfg, comm->num_sms, s, dry);
   }
   Args<double, int32_t> a;
-  fill_args(B, a, io, kmax, rtol, 0.0, cfg, dry);
+  fill_args(B, a, io, kmax, rtol, delta2_of(B, prec), cfg, dry);
   return launch_f64(&a, false, cfg, comm->num_sms, s, dry);
+}
+
+// The solve with every unit in its own group of CTAs (batch_onchip.cu); false
+// when the batch does not fit that form (nothing has been launched).
+bool run_onchip(spmv_batch B, spmv_batch_precision prec, const SolveIo& io, int kmax,
+                double rtol) {
+  spmv_comm comm = B->comm;
+  cudaStream_t s = comm->stream;
+  const bool fp32 = prec == SPMV_BATCH_MIXED;
+  const int nrhs = io.with_block ? B->block_nrhs : 0;
+  spmv_batch_s::Onchip& oc = B->oc[prec][io.with_block ? 1 : 0];
+  if (!oc.planned) {
+    plan_onchip(B->plan, B->block_sys, nrhs, fp32, comm->device, comm->num_sms, oc.plan);
+    if (oc.plan.ok) upload(oc.ctas, oc.plan.ctas.data(), sizeof(OnchipCta) * oc.plan.ctas.size());
+    oc.planned = true;
+  }
+  const OnchipPlan& p = oc.plan;
+  if (!p.ok) return false;
+  B->oc_p.reserve((fp32 ? sizeof(float) : sizeof(double)) * size_t(p.rows));
+  B->oc_x.reserve(sizeof(double) * size_t(p.rows));
+  B->oc_b.reserve(sizeof(double) * size_t(p.rows));
+  B->oc_parts.reserve(sizeof(double) * size_t(p.parts));
+  const size_t bars = sizeof(unsigned long long) * OC_BAR * size_t(p.nbars);
+  B->oc_bars.reserve(bars);
+  SPMVB_CUDA(cudaMemsetAsync(B->oc_bars.ptr, 0, bars, s));
+  SPMVB_CUDA(cudaMemsetAsync(B->err.ptr, 0, sizeof(int), s));
+  OnchipArgs a{};
+  a.vals = fp32 ? B->vals32.ptr : B->vals64.ptr;
+  a.idx = B->idx.ptr;
+  a.vals64 = B->vals64.as<double>();
+  a.items = B->oc_items.as<int4>();
+  a.perm = B->perm.as<int32_t>();
+  a.ctas = oc.ctas.as<OnchipCta>();
+  a.p = B->oc_p.ptr;
+  a.x = B->oc_x.as<double>();
+  a.b = B->oc_b.as<double>();
+  a.b_user = io.b_user;
+  a.x_user = io.x_user;
+  a.B_user = io.B_user;
+  a.X_user = io.X_user;
+  a.slots = B->slots.as<Slot>();
+  a.parts = B->oc_parts.as<double>();
+  a.bars = B->oc_bars.as<unsigned long long>();
+  a.err = B->err.as<int>();
+  a.limit_ns = wait_ns();
+  a.rtol2 = rtol * rtol;
+  a.delta2 = delta2_of(B, prec);
+  a.kmax = kmax;
+  a.nrhs = nrhs;
+  a.per_warp = p.per_warp;
+  a.alloc = p.alloc;
+  // Half of L2 (24 systems of 22,000 rows, 46 MB: 13.1 us per iteration kept,
+  // 15.1 streamed; larger batches would push each other and p out).
+  int l2 = 0;
+  SPMVB_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, comm->device));
+  a.keep = B->plan.entries * int64_t((fp32 ? 4 : 8) + (B->plan.fits16 ? 2 : 4)) <= l2 / 2;
+  return launch_onchip(p, a, s);
 }
 
 // The configured shape, or 1 CTA per SM when 2 do not fit.
@@ -387,6 +457,16 @@ int spmv_batch_create(spmv_comm comm, int nsys, const int32_t* n,
     else
       upload(B->idx, P.col32.data(), sizeof(int32_t) * P.col32.size());
     upload(B->perm, P.perm.data(), sizeof(int32_t) * P.perm.size());
+    {
+      std::vector<int4> items(size_t(P.nslices));
+      for (int i = 0; i < nsys; ++i)
+        for (int64_t k = 0; k < (P.n[i] + 31) / 32; ++k) {
+          const int64_t g = P.slice0[i] + k;
+          const int64_t w = (P.soff[g + 1] - P.soff[g]) / 32;
+          items[size_t(g)] = make_int4(int(P.soff[g] / 32), int(32 * k), int(w) | 32 << 24, 0);
+        }
+      upload(B->oc_items, items.data(), sizeof(int4) * items.size());
+    }
     // The host copies of the big arrays are not needed again.
     std::vector<float>().swap(P.vals32);
     std::vector<double>().swap(P.vals64);
@@ -394,7 +474,6 @@ int spmv_batch_create(spmv_comm comm, int nsys, const int32_t* n,
     std::vector<int32_t>().swap(P.col32);
     std::vector<int32_t>().swap(P.perm);
     std::vector<int64_t>().swap(P.soff);
-    std::vector<int32_t>().swap(P.sbound);
     const int64_t rows = std::max<int64_t>(P.rows_pad, 32);
     B->x.reserve(sizeof(double) * rows);
     B->b.reserve(sizeof(double) * rows);
@@ -498,6 +577,7 @@ int spmv_batch_set_block(spmv_batch B, int system, int nrhs) {
     B->block_npad = npad;
     B->block_nnz = int64_t(bc.size());
     build_units(B);
+    for (auto& o : B->oc) o[1].planned = false;
   });
 }
 
@@ -506,6 +586,7 @@ int spmv_batch_set_config(spmv_batch B, spmv_batch_precision prec, const spmv_ba
     require(B != nullptr && c != nullptr, "spmv: NULL argument");
     require(prec == SPMV_BATCH_MIXED || prec == SPMV_BATCH_FP64, "spmv batch: unknown precision");
     LaunchCfg& cfg = B->cfg[prec];
+    if (c->ctas_per_sm || c->tile_rows || c->rhs_lanes || c->window) cfg.chosen = true;
     if (c->ctas_per_sm) {
       require(c->ctas_per_sm == 1 || c->ctas_per_sm == 2, "spmv batch: ctas_per_sm must be 1 or 2");
       cfg.cps = c->ctas_per_sm;
@@ -715,9 +796,15 @@ int spmv_batch_solve_ex(spmv_batch B, spmv_memory memory, spmv_batch_precision p
     io.B_user = blk ? Bd : nullptr;
     io.X_user = blk ? Xd : nullptr;
     io.with_block = blk;
-    const LaunchCfg cfg = resident_cfg(B, precision, B->cfg[precision], io);
-    require(run(B, precision, io, max_its, rtol, cfg, false),
-            "spmv batch: the kernel cannot be made resident");
+    // The on-chip form where the batch fits it, unless the caller chose the
+    // lockstep kernel's shape or asks for its phase times.
+    const bool onchip = !B->cfg[precision].chosen && !std::getenv("SPMV_B200_BATCH_PROFILE") &&
+                        run_onchip(B, precision, io, max_its, rtol);
+    if (!onchip) {
+      const LaunchCfg cfg = resident_cfg(B, precision, B->cfg[precision], io);
+      require(run(B, precision, io, max_its, rtol, cfg, false),
+              "spmv batch: the kernel cannot be made resident");
+    }
     const int nslot = ns + (blk ? BW : 0);
     std::vector<Slot> sl(std::max(nslot, 1));
     if (nslot)
@@ -737,6 +824,13 @@ int spmv_batch_solve_ex(spmv_batch B, spmv_memory memory, spmv_batch_precision p
     }
     SPMVB_CUDA(cudaStreamSynchronize(s));
     check_err(B);
+    if (onchip)  // an empty system has no CTA
+      for (int i = 0; i < nslot; ++i)
+        if (P.n[i < ns ? i : B->block_sys] == 0) {
+          sl[i] = Slot{};
+          sl[i].status = SPMV_SUCCESS;
+          sl[i].converged = 1;
+        }
     write_profile(B, precision == SPMV_BATCH_MIXED ? "mixed" : "fp64");
     auto fill = [](const Slot& q, spmv_batch_info& o) {
       o.iterations = q.its;

@@ -114,13 +114,14 @@ struct Plan {
   std::vector<int64_t> row0, slice0; // per system
   // Host copies (uploaded, then freed).
   std::vector<int64_t> soff;
-  std::vector<int32_t> sbound;       // 2 per slice: min and max unit-local column
   std::vector<float> vals32;
   std::vector<double> vals64;
   std::vector<int16_t> off16;
   std::vector<int32_t> col32;
   std::vector<int32_t> perm;
   std::vector<std::vector<int32_t>> sys_perm;  // per system: new -> old row
+  std::vector<int32_t> sbound;       // 2 per slice: min and max unit-local column
+  std::vector<int64_t> sys_entries;  // per system: stored entries (with padding)
 };
 
 // Host planning of one batch: per system a reverse Cuthill-McKee order,
@@ -137,6 +138,7 @@ struct LaunchCfg {
   int tile_slices = 8;   // rows per warp tile: 32 x tile_slices (single units)
   int rhs_rows = 1;      // block rows per warp step (lanes per row 32 / rhs_rows)
   int window = 1;        // products stage the gathered vector in shared memory
+  bool chosen = false;   // set by the caller: solves use the lockstep kernel
 };
 
 // Launch of the lockstep kernel (cooperative; the grid must be resident):
@@ -146,6 +148,63 @@ bool launch_f32(const void* args, bool d16, const LaunchCfg& c, int num_sms, cud
                 bool dry);
 bool launch_f64(const void* args, bool d16, const LaunchCfg& c, int num_sms, cudaStream_t s,
                 bool dry);
+
+// One CTA of the on-chip kernel (batch_onchip.cu): slices of a unit's matrix and
+// its place in the unit's group.
+struct OnchipCta {
+  int64_t item0;   // first slice in the slice table
+  int64_t vec0;    // the unit's first row in x, b and p
+  int64_t perm0;   // and in perm
+  int64_t part0;   // the group's partial sums
+  int32_t nitems;  // slices
+  int32_t g0;      // first row (of the unit)
+  int32_t w0, wrows;  // rows of p in shared memory (whole slices, the CTA's included)
+  int32_t full;       // every column of the CTA's slices is one of them
+  int32_t bar;     // the group's counter
+  int32_t rank, size;
+  int32_t sys, col, slot;  // col -1: the system's own right-hand side
+};
+constexpr int OC_BAR = 16;  // counters per barrier (one 128-byte line each)
+
+struct OnchipPlan {
+  bool ok = false;
+  const void* fn = nullptr;
+  int per_warp = 0;        // slices per warp at most
+  int alloc = 0;           // tensor-memory columns
+  int64_t smem = 0, rows = 0, parts = 0;
+  int nbars = 0;
+  std::vector<OnchipCta> ctas;
+};
+
+struct OnchipArgs {
+  const void* vals;        // inner-precision values
+  const void* idx;
+  const double* vals64;
+  const int4* items;       // per slice: first entry / 32, first row, columns | 32 << 24
+  const int32_t* perm;
+  const OnchipCta* ctas;
+  void* p;
+  double *x, *b;
+  const double* const* b_user;
+  double* const* x_user;
+  const double* B_user;
+  double* X_user;
+  Slot* slots;
+  double* parts;
+  unsigned long long* bars;  // [0]: the grid's
+  int* err;
+  unsigned long long limit_ns;
+  double rtol2, delta2;
+  int kmax, nrhs, per_warp, alloc;
+  bool keep;  // the matrices fit in L2 with room to spare
+};
+
+// Groups of CTAs for the batch's systems (and nrhs columns of block_sys); false
+// when there are more units than SMs or their rows do not fit on chip.
+bool plan_onchip(const Plan& P, int block_sys, int nrhs, bool fp32, int device, int num_sms,
+                 OnchipPlan& out);
+// False when the grid cannot be resident.
+bool launch_onchip(const OnchipPlan& plan, OnchipArgs& a, cudaStream_t s);
 
 }  // namespace bat
 }  // namespace spmvb

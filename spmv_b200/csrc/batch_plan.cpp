@@ -175,6 +175,7 @@ void plan_batch(int nsys, const int32_t* n, const int32_t* const* rowptr,
   for (int s = 0; s < nsys; ++s) {
     P.nnz[s] = rowptr[s][n[s]];
     P.nnz_total += P.nnz[s];
+    P.sys_entries.push_back(lay[s].entries);
     P.row0[s] = rows;
     P.slice0[s] = slices;
     rows += 32 * int64_t(lay[s].sw.size());

@@ -503,7 +503,9 @@ __device__ __forceinline__ int warp_total_of() {
 
 // N sums at once: parts holds N partials per CTA (CTA b's at parts[N b .. N b
 // + N - 1]); every thread of every CTA gets the same N totals, in a fixed order
-// (lanes, warps, then CTAs by lane, lanes, warps).  No
+// (lanes, warps, then CTAs by lane, lanes, warps).  The CTAs are the grid, or a
+// group of `size` of them with its own parts and counter (rank: the CTA's place
+// in it).  No
 // step is serial over warps or CTAs, as coop_grid_sum_n's are: a sum of four at
 // 148 CTAs of 24 warps took 4.1 us that way, of which 1.5 are the barrier, and
 // takes 2.9 this way.  (With 12 warps and 296 or 444 CTAs the serial steps are
@@ -524,7 +526,9 @@ __device__ __forceinline__ bool coop_grid_totals(const double (&v)[N], double* p
                                                 unsigned long long* count,
                                                 unsigned long long target, int* err,
                                                 unsigned long long limit_ns, GridTotals<NT, N>& s,
-                                                double (&total)[N]) {
+                                                double (&total)[N],
+                                                const unsigned int rank = blockIdx.x,
+                                                const unsigned int size = gridDim.x) {
   constexpr int NW = NT / 32;
   static_assert(NW <= 32, "one lane per warp");
   const int warp = int(threadIdx.x) >> 5, lane = int(threadIdx.x) & 31;
@@ -539,9 +543,11 @@ __device__ __forceinline__ bool coop_grid_totals(const double (&v)[N], double* p
 #pragma unroll
     for (int j = 0; j < N; ++j) w[j] = lane < NW ? s.red[j][lane] : 0.0;
     const double x = warp_totals<N>(w);
-    if (mine >= 0) __stcg(parts + N * blockIdx.x + mine, x);
+    if (mine >= 0) __stcg(parts + N * rank + mine, x);
     __syncwarp();
-    if (lane == 0) s.ok = grid_arrive_wait(count, target, err, limit_ns);
+    if (lane == 0)
+      s.ok = size == 1u ? *static_cast<volatile int*>(err) == 0
+                        : grid_arrive_wait(count, target, err, limit_ns);
   }
   named_sync(1, NT);
   if (!s.ok) return false;
@@ -551,7 +557,7 @@ __device__ __forceinline__ bool coop_grid_totals(const double (&v)[N], double* p
   if (j < N) {
     double x = 0.0;
 #pragma unroll 2
-    for (unsigned int b = 32u * unsigned(q) + unsigned(lane); b < gridDim.x; b += 32u * PV)
+    for (unsigned int b = 32u * unsigned(q) + unsigned(lane); b < size; b += 32u * PV)
       x += __ldcg(parts + N * b + j);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);

@@ -44,6 +44,7 @@ struct RingView {
   int count, stride;    // items of the CTA; the warp takes warp, warp + stride, ...
   unsigned char* base;  // the warp's slots
   uint64_t* bar;        // and their barriers
+  bool keep = false;    // L2 should hold the entries from one pass to the next
 };
 
 // State of a warp's ring (registers).
@@ -75,7 +76,7 @@ __device__ __forceinline__ void ring_issue(const RingView<T, CI>& v, RingState& 
     uint64_t* bar = v.bar + r.fill;
     mbar_arrive_expect_tx(bar, n * uint32_t(sizeof(T) + sizeof(CI)));
     if (n > 0) {
-      const uint64_t policy = l2_policy_stream();
+      const uint64_t policy = v.keep ? l2_policy_keep() : l2_policy_stream();
       bulk_g2s(s, v.vals + e, n * uint32_t(sizeof(T)), bar, policy);
       bulk_g2s(s + Sh::VB, v.idx + e, n * uint32_t(sizeof(CI)), bar, policy);
     }
@@ -258,6 +259,19 @@ __device__ __forceinline__ void tmem_ld(uint32_t addr, Tmem64& a) {
 __device__ __forceinline__ void tmem_st(uint32_t addr, double v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(addr),
                "r"(__double2loint(v)), "r"(__double2hiint(v))
+               : "memory");
+}
+// 32-bit values in one column.
+struct Tmem32 {
+  uint32_t v;
+  __device__ __forceinline__ float get() const { return __uint_as_float(v); }
+};
+__device__ __forceinline__ void tmem_ld(uint32_t addr, Tmem32& a) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(a.v) : "r"(addr));
+}
+__device__ __forceinline__ void tmem_st(uint32_t addr, float v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(addr),
+               "r"(__float_as_uint(v))
                : "memory");
 }
 
