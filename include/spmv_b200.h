@@ -341,7 +341,8 @@ int spmv_matrix_cg_form(spmv_matrix A, int* fused, int* ctas_per_sm, int* r_shar
 
 /* The same for spmv_cg_mixed: *fused = 0 for its CUDA graph (three kernels
  * per inner iteration, three more per refinement), 1 for one cooperative
- * launch per solve (the FP32 residual in shared memory when *r_shared = 1).
+ * launch per solve (the FP32 residual in shared memory when *r_shared = 1),
+ * 2 for its merged-update form with the vectors on chip (*r_shared = 2).
  * Fails when spmv_cg_mixed has not run on the matrix.  No reference
  * counterpart. */
 int spmv_matrix_cg_mixed_form(spmv_matrix A, int* fused, int* ctas_per_sm, int* r_shared);

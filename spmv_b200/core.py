@@ -384,7 +384,7 @@ class Matrix:
         """How cg (solver="cg") or cg_mixed (solver="mixed") runs on this
         matrix: ("graph", 0, None) for its kernels in a CUDA graph, or
         ("fused", CTAs per SM, "smem", "tmem" or "global": where the residual
-        lives) for one cooperative launch per solve, with ":m" appended for cg's
+        lives) for one cooperative launch per solve, with ":m" appended for the
         merged-update form (two grid syncs per iteration); fails if that
         solver has not run on the matrix."""
         fn = {"cg": "spmv_matrix_cg_form", "mixed": "spmv_matrix_cg_mixed_form"}[solver]

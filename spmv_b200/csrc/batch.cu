@@ -304,7 +304,7 @@ bool run(spmv_batch B, spmv_batch_precision prec, const SolveIo& io, int kmax, d
   return launch_f64(&a, false, cfg, comm->num_sms, s, dry);
 }
 
-// The solve with every unit in its own group of CTAs (batch_onchip.cu); false
+// The solve with every unit in its own group of CTAs (onchip.cu); false
 // when the batch does not fit that form (nothing has been launched).
 bool run_onchip(spmv_batch B, spmv_batch_precision prec, const SolveIo& io, int kmax,
                 double rtol) {

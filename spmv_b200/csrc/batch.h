@@ -149,7 +149,7 @@ bool launch_f32(const void* args, bool d16, const LaunchCfg& c, int num_sms, cud
 bool launch_f64(const void* args, bool d16, const LaunchCfg& c, int num_sms, cudaStream_t s,
                 bool dry);
 
-// One CTA of the on-chip kernel (batch_onchip.cu): slices of a unit's matrix and
+// One CTA of the on-chip kernel (onchip.cu): slices of a unit's matrix and
 // its place in the unit's group.
 struct OnchipCta {
   int64_t item0;   // first slice in the slice table
@@ -158,7 +158,8 @@ struct OnchipCta {
   int64_t part0;   // the group's partial sums
   int32_t nitems;  // slices
   int32_t g0;      // first row (of the unit)
-  int32_t w0, wrows;  // rows of p in shared memory (whole slices, the CTA's included)
+  int32_t rows;    // its rows
+  int32_t w0, wrows;  // rows of p in shared memory (the CTA's included; multiples of 4)
   int32_t full;       // every column of the CTA's slices is one of them
   int32_t bar;     // the group's counter
   int32_t rank, size;
@@ -169,6 +170,7 @@ constexpr int OC_BAR = 16;  // counters per barrier (one 128-byte line each)
 struct OnchipPlan {
   bool ok = false;
   const void* fn = nullptr;
+  int block = 0;           // threads per CTA
   int per_warp = 0;        // slices per warp at most
   int alloc = 0;           // tensor-memory columns
   int64_t smem = 0, rows = 0, parts = 0;
@@ -203,6 +205,9 @@ struct OnchipArgs {
 // when there are more units than SMs or their rows do not fit on chip.
 bool plan_onchip(const Plan& P, int block_sys, int nrhs, bool fp32, int device, int num_sms,
                  OnchipPlan& out);
+// One group over the grid for a matrix's mixed solve (FP32 inner; SELL layout with
+// FP32 values built); false when its rows do not fit on chip.
+bool plan_onchip_matrix(spmv_matrix A, OnchipPlan& out);
 // False when the grid cannot be resident.
 bool launch_onchip(const OnchipPlan& plan, OnchipArgs& a, cudaStream_t s);
 

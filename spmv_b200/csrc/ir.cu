@@ -29,6 +29,7 @@
 
 #include <type_traits>
 
+#include "batch.h"
 #include "internal.h"
 #include "sell_staged.cuh"
 #include "spmv_kernel.cuh"
@@ -56,6 +57,12 @@ struct IrWorkspace {
   int fused_grid = 0, fused_block = 0, fused_smem = 0, fused_cps = 0;
   bool fused_rs = false;
   spmvb::DevBuf bar, fpartials, ctas;
+  // The on-chip form (onchip.cu): its plan, result and arguments.
+  bool fused_tm = false;
+  spmvb::bat::OnchipPlan onchip;
+  spmvb::bat::OnchipArgs oargs{};
+  spmvb::DevBuf oslot;
+  spmvb::bat::Slot hslot{};
   spmvb::SpmvArgs fa32, fa64;  // FP32 product over p, FP64 SELL over x
   IrState host{};
   ~IrWorkspace() {
@@ -970,6 +977,7 @@ bool ir_plan(spmv_matrix A, const IrWorkspace& w, FusedPlan& plan) {
 
 void ir_use_plan(IrWorkspace& w, const FusedPlan& plan) {
   w.fused = true;
+  w.fused_tm = false;
   w.fused_fn = plan.fn;
   w.fused_grid = plan.grid;
   w.fused_block = plan.block;
@@ -982,6 +990,34 @@ void ir_use_plan(IrWorkspace& w, const FusedPlan& plan) {
                         cudaMemcpyHostToDevice));
 }
 
+// The on-chip form, if the matrix fits it.
+bool ir_use_onchip(spmv_matrix A, IrWorkspace& w) {
+  bat::OnchipPlan& p = w.onchip;
+  if (!bat::plan_onchip_matrix(A, p)) return false;
+  w.fused = w.fused_tm = true;
+  w.fused_cps = 1;
+  w.fused_rs = true;
+  w.fused_grid = int(p.ctas.size());
+  w.fpartials.reserve(sizeof(double) * size_t(p.parts));
+  w.oslot.reserve(sizeof(bat::Slot));
+  w.ctas.reserve(sizeof(bat::OnchipCta) * p.ctas.size());
+  SPMVB_CUDA(cudaMemcpy(w.ctas.ptr, p.ctas.data(), sizeof(bat::OnchipCta) * p.ctas.size(),
+                        cudaMemcpyHostToDevice));
+  const DevCsr& C = A->fwd;
+  bat::OnchipArgs a{};
+  a.vals = C.sell_vals32.ptr;
+  a.vals64 = C.sell_vals.as<double>();
+  a.idx = C.d16 ? C.sell_d16_global.ptr : C.sell_cols_global.ptr;
+  a.items = item_table(A, 1).desc.as<int4>();
+  a.p = w.p.ptr;
+  a.x = w.x.as<double>();
+  a.b = w.b.as<double>();
+  a.per_warp = p.per_warp;
+  a.alloc = p.alloc;
+  w.oargs = a;
+  return true;
+}
+
 // One solve as ir_run enqueues it: kmax, rtol^2, delta^2 and the error
 // flag, then the fused launch or the graph.
 void ir_enqueue(IrWorkspace& w, cudaStream_t s) {
@@ -989,6 +1025,27 @@ void ir_enqueue(IrWorkspace& w, cudaStream_t s) {
   SPMVB_CUDA(cudaMemcpyAsync(&st->kmax, &w.host.kmax, sizeof(int), cudaMemcpyHostToDevice, s));
   SPMVB_CUDA(cudaMemcpyAsync(&st->rtol2, &w.host.rtol2, 2 * sizeof(double),
                              cudaMemcpyHostToDevice, s));
+  if (w.fused_tm) {
+    const size_t g = size_t(w.fused_grid);
+    require(w.fpartials.bytes >= 8 * g * sizeof(double) &&
+                w.ctas.bytes >= g * sizeof(bat::OnchipCta),
+            "spmv: on-chip mixed CG buffers smaller than its grid");
+    SPMVB_CUDA(cudaMemsetAsync(&st->stage_err, 0, sizeof(int), s));
+    SPMVB_CUDA(cudaMemsetAsync(w.bar.ptr, 0, sizeof(unsigned long long), s));
+    bat::OnchipArgs a = w.oargs;
+    a.ctas = w.ctas.as<bat::OnchipCta>();
+    a.slots = w.oslot.as<bat::Slot>();
+    a.parts = w.fpartials.as<double>();
+    a.bars = w.bar.as<unsigned long long>();
+    a.err = &st->stage_err;
+    a.kmax = w.host.kmax;
+    a.rtol2 = w.host.rtol2;
+    a.delta2 = w.host.delta2;
+    a.limit_ns = fused_wait_ns();
+    if (bat::launch_onchip(w.onchip, a, s)) return;
+    // (A grid that no longer fits on the device: the graph form from here on.)
+    w.fused = w.fused_tm = false;
+  }
   if (w.fused) {
     const size_t g = size_t(w.fused_grid);
     require(w.fpartials.bytes >= 6 * g * sizeof(double) &&
@@ -1055,12 +1112,17 @@ float ir_time(IrWorkspace& w, cudaStream_t s, int its) {
 // cap forces), scored s + F / 100: solves to 1e-10 refine about once per
 // 50..250 inner iterations.  The candidates are two
 // CTAs per SM of 3 stages with r in shared or global memory, or three of 4
-// stages (the graph form's product shape) with r in global memory.
-// SPMV_B200_CG_MIXED_FUSED: "0" keeps the graph form; "2:smem", "2:global"
-// or "3:global" forces that plan, failing if it does not fit.
+// stages (the graph form's product shape) with r in global memory; or the
+// on-chip form, for any matrix with the SELL layout.
+// SPMV_B200_CG_MIXED_FUSED: "0" keeps the graph form; "2:smem", "2:global",
+// "3:global" or "1:tmem:m" forces that plan, failing if it does not fit.
 void ir_choose_form(spmv_matrix A, IrWorkspace& w) {
-  w.fused = false;
-  if (w.p32.kind != ProductKind::Staged || w.n == 0) return;
+  w.fused = w.fused_tm = false;
+  if (w.n == 0) return;
+  const bool onchip = A->fwd.sell_cols_global.ptr != nullptr && A->fwd.sell_vals32.ptr != nullptr &&
+                      (!A->kernel_set || A->kernel == SPMV_KERNEL_STAGED);
+  const bool staged = w.p32.kind == ProductKind::Staged;
+  if (!onchip && !staged) return;
   const char* env = std::getenv("SPMV_B200_CG_MIXED_FUSED");
   const std::string mode = env ? env : "";
   if (mode == "0") return;
@@ -1068,30 +1130,46 @@ void ir_choose_form(spmv_matrix A, IrWorkspace& w) {
   int coop = 0;
   SPMVB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, comm->device));
   if (!coop) return;
-  if (!ir_tiles(A, w.p32, true).ok) return;
+  const bool tiles = staged && ir_tiles(A, w.p32, true).ok;
+  if (!onchip && !tiles) return;
   w.bar.reserve(sizeof(unsigned long long));
-  ir_args(A, w, w.p32, true, w.fa32);
-  SolverProduct s64 = w.p32;  // the FP64 residual walks the same SELL slices
-  ir_args(A, w, s64, false, w.fa64);
+  if (tiles) {
+    ir_args(A, w, w.p32, true, w.fa32);
+    SolverProduct s64 = w.p32;  // the FP64 residual walks the same SELL slices
+    ir_args(A, w, s64, false, w.fa64);
+  }
   if (!mode.empty()) {
     FusedPlan p;
     bool fits = false;
-    if (mode == "2:smem") fits = ir_plan<IrFusedTwo, true>(A, w, p);
+    if (mode == "1:tmem:m" && onchip && ir_use_onchip(A, w)) return;
+    if (!tiles) fits = false;
+    else if (mode == "2:smem") fits = ir_plan<IrFusedTwo, true>(A, w, p);
     else if (mode == "2:global") fits = ir_plan<IrFusedTwo, false>(A, w, p);
     else if (mode == "3:global") fits = ir_plan<IrFusedThree, false>(A, w, p);
     require(fits, "spmv: SPMV_B200_CG_MIXED_FUSED must be 0 or a fused plan that fits this "
-                  "matrix (2:smem, 2:global, 3:global)");
+                  "matrix (2:smem, 2:global, 3:global, 1:tmem:m)");
     ir_use_plan(w, p);
     return;
   }
+  // Where every CTA's window of p fits, the other forms have not been faster (us
+  // per inner iteration, on chip, the best other fused plan, graph: 27-point 96^3
+  // 30.5, 41.3, 51.8; 40^3 8.2, 10.7, 24.7; 7-point 64^3 8.7, 11.3, 24.8; 5-point
+  // 1024^2 14.5, 17.3, 30.5; 1400^2 22.3, 25.4, 38.6), so nothing is timed.  Where
+  // one does not (7-point 128^3: 33.0, 31.2, 44.8), every plan that fits is.
+  if (onchip && ir_use_onchip(A, w)) {
+    bool full = true;
+    for (const bat::OnchipCta& c : w.onchip.ctas) full = full && c.full;
+    if (full) return;
+    w.fused = w.fused_tm = false;
+  }
   std::vector<FusedPlan> plans;
-  {
+  if (tiles) {
     FusedPlan p1, p2, p3;
     if (ir_plan<IrFusedTwo, true>(A, w, p1)) plans.push_back(std::move(p1));
     if (ir_plan<IrFusedTwo, false>(A, w, p2)) plans.push_back(std::move(p2));
     if (ir_plan<IrFusedThree, false>(A, w, p3)) plans.push_back(std::move(p3));
   }
-  if (plans.empty()) return;
+  if (plans.empty() && !onchip) return;
   cudaStream_t s = comm->stream;
   SPMVB_CUDA(cudaDeviceSynchronize());
   ir_fill<<<std::max(1, comm->num_sms) * 4, 256, 0, s>>>(w.b.as<double>(), w.n, 1.0);
@@ -1106,6 +1184,12 @@ void ir_choose_form(spmv_matrix A, IrWorkspace& w) {
   };
   float best = score("graph");
   int pick = -1;
+  bool chip = false;
+  if (onchip && ir_use_onchip(A, w)) {
+    const float t = score("on chip");
+    chip = w.fused_tm && t < best;
+    if (chip) best = t;
+  }
   for (size_t i = 0; i < plans.size(); ++i) {
     ir_use_plan(w, plans[i]);
     const std::string name = "fused " + std::to_string(plans[i].cps) +
@@ -1117,8 +1201,11 @@ void ir_choose_form(spmv_matrix A, IrWorkspace& w) {
       pick = int(i);
     }
   }
-  w.fused = false;
-  if (pick >= 0) ir_use_plan(w, plans[size_t(pick)]);
+  w.fused = w.fused_tm = false;
+  if (pick >= 0)
+    ir_use_plan(w, plans[size_t(pick)]);
+  else if (chip)
+    ir_use_onchip(A, w);
 }
 
 }  // namespace
@@ -1148,12 +1235,12 @@ IrWorkspace& ir_workspace(spmv_matrix A) {
     w->x.reserve(8 * n1);
     w->r64.reserve(8 * n1);
     w->r.reserve(4 * n1);
-    w->p.reserve(4 * n1);
+    w->p.reserve(4 * n1 + 16);  // read in groups of four
     w->y.reserve(4 * n1);
     w->d.reserve(4 * n1);
     w->state.reserve(sizeof(IrState));
     SPMVB_CUDA(cudaMemset(w->state.ptr, 0, sizeof(IrState)));
-    SPMVB_CUDA(cudaMemset(w->p.ptr, 0, 4 * n1));
+    SPMVB_CUDA(cudaMemset(w->p.ptr, 0, 4 * n1 + 16));
     SPMVB_CUDA(cudaMemset(w->x.ptr, 0, 8 * n1));
     // Each product (FP32 inner, FP64 residual) is the candidate whose own
     // kernel (timed outside the graph) is fastest on this matrix; the FP64
@@ -1210,6 +1297,7 @@ CgForm ir_form(spmv_matrix A) {
   f.fused = w.fused;
   f.cps = w.fused ? w.fused_cps : 0;
   f.rs = w.fused && w.fused_rs;
+  f.merged = f.tmem = w.fused && w.fused_tm;
   return f;
 }
 
@@ -1230,9 +1318,20 @@ void ir_run(spmv_matrix A, int max_its, double rtol, spmv_ir_info* info) {
   w.host.delta2 = 0.01;  // refine when ||r|| fell 10x below its recent maximum
   ir_enqueue(w, s);
   SPMVB_CUDA(cudaMemcpyAsync(&w.host, st, sizeof(IrState), cudaMemcpyDeviceToHost, s));
+  const bool tm = w.fused_tm;
+  if (tm)
+    SPMVB_CUDA(cudaMemcpyAsync(&w.hslot, w.oslot.ptr, sizeof(bat::Slot), cudaMemcpyDeviceToHost, s));
   SPMVB_CUDA(cudaStreamSynchronize(s));
   if (w.host.stage_err)
     fail(SPMV_ERROR_CUDA, "spmv: a bounded wait on the device timed out");
+  if (tm) {
+    w.host.k = w.hslot.its;
+    w.host.refinements = w.hslot.refs;
+    w.host.status = w.hslot.status;
+    w.host.converged = w.hslot.converged;
+    w.host.rr0 = w.hslot.rr0;
+    w.host.rr_true = w.hslot.rr_true;
+  }
   if (info) {
     info->iterations = w.host.k;
     info->refinements = w.host.refinements;

@@ -1,8 +1,9 @@
-// Batched CG with the vectors on chip (no counterpart in the reference; each
-// recurrence is spmv::cg's, cg.cpp:50-80, with the FP32-inner / FP64-refinement
-// scheme of the mixed solver).
+// CG with the vectors on chip for the batched and the mixed solves (no counterpart
+// in the reference; each recurrence is spmv::cg's, cg.cpp:50-80, with the
+// FP32-inner / FP64-refinement scheme of the mixed solver).  The mixed solve of one
+// matrix is one group over the grid, on the matrix's SELL layout (MX below).
 //
-// Every unit (a system, or one column of the block of right-hand sides) gets
+// In a batch every unit (a system, or one column of the block of right-hand sides) gets
 // its own group of CTAs of one cooperative launch, and the groups iterate
 // independently: each has its own counter and partial sums, so nothing waits for
 // a larger unit, and a unit that has converged leaves.  A CTA keeps its rows' p
@@ -36,6 +37,10 @@
 // small systems: 5 us with one CTA, 7 with more.  7 systems of 800 to 3,000 rows
 // and 5 columns: 63 us in the lockstep kernel, 5.6 here; 24 of 22,000 and 32
 // columns, the chip full, 105 and 24.
+// One matrix, mixed (the fused form of ir.cu before): 27-point 96^3 41.3 us per
+// iteration, now 30.5 (of which its entries are 22 at the rate of a copy); 5-point
+// 1024^2 17.3 and 14.5, 200 x 180 19.1 and 5.8 (as a CUDA graph before); 27-point
+// 40^3 10.7 and 8.2.
 #include <algorithm>
 #include <cmath>
 #include <queue>
@@ -55,6 +60,14 @@ namespace {
 constexpr int OC_NW = 20;
 constexpr int OC_U = 16;
 constexpr int OC_D = 1;
+
+// The same for one matrix over the grid, whose entries come from memory: more
+// warps and copies in flight (us per iteration, 27-point 96^3 / 5-point 1024^2 /
+// 7-point 128^3: 28 warps 9 x 2 30.5 / 14.5 / 33.0; 24 warps 9 x 2 30.5 / 15.4 / 36.9;
+// 20 warps 9 x 3 30.8 / 15.7 / 40.7, 14 x 2 30.7 / 15.9 / 41.7, 16 x 1 34.5 / 18.3 / 46.2).
+constexpr int OCM_NW = 28;
+constexpr int OCM_U = 9;
+constexpr int OCM_D = 2;
 
 struct OcScalars {
   double rr0, rr_max, rr_true, rr_prev, alpha, beta, s, c;
@@ -114,29 +127,37 @@ __device__ __forceinline__ double oc_fma(double a, double b, double c) {
   return __fma_rn(a, b, c);
 }
 
+// A matrix's padding entries (value 0; the batch's have the row's own column).
+template <typename CI>
+__device__ __forceinline__ bool oc_padding(int c) {
+  return sizeof(CI) == 2 ? c == -32768 : c < 0;
+}
+
 // The first W columns of a landed slot (vals, idx: the lane's entries): sum += v
 // p.  pl: p in shared memory (as the lane's column 0 or, with 16-bit offsets, its
 // row), pg: the same place in the unit's p, at row l of the window of `rows`; FULL:
 // the window holds every column.
-template <int W, bool FULL, typename T, typename CI>
+template <int W, bool FULL, bool MX, typename T, typename CI>
 __device__ __forceinline__ void oc_slot(const T* vals, const CI* idx, const T* pl, const T* pg,
                                         int l, unsigned rows, T& sum) {
   T x[W];
 #pragma unroll
   for (int u = 0; u < W; ++u) {
     const int c = int(idx[32 * u]);
-    x[u] = FULL || unsigned(l + c) < rows ? pl[c] : __ldcg(pg + c);
+    x[u] = T(0);
+    if (!MX || !oc_padding<CI>(c))
+      x[u] = FULL || unsigned(l + c) < rows ? pl[c] : __ldcg(pg + c);
   }
 #pragma unroll
   for (int u = 0; u < W; ++u) sum = oc_fma(vals[32 * u], x[u], sum);
 }
-template <int W, bool FULL, typename T, typename CI>
+template <int W, bool FULL, bool MX, typename T, typename CI>
 __device__ __forceinline__ void oc_slot_of(int w, const T* vals, const CI* idx, const T* pl,
                                            const T* pg, int l, unsigned rows, T& sum) {
   if (w == W)
-    oc_slot<W, FULL>(vals, idx, pl, pg, l, rows, sum);
+    oc_slot<W, FULL, MX>(vals, idx, pl, pg, l, rows, sum);
   else if constexpr (W > 1)
-    oc_slot_of<W - 1, FULL>(w, vals, idx, pl, pg, l, rows, sum);
+    oc_slot_of<W - 1, FULL, MX>(w, vals, idx, pl, pg, l, rows, sum);
 }
 
 // ring_pass for this layout, whose entries are all stored ones (padding is the
@@ -144,7 +165,7 @@ __device__ __forceinline__ void oc_slot_of(int w, const T* vals, const CI* idx, 
 // columns.  A pass is bound by the instructions it issues (FP32, 24 systems of
 // 22,000 rows of 14 entries: 49 per 32 entries with ring_pass's masks and its test
 // of every column against the window).
-template <bool FULL, typename T, typename CI, int U, int D, class F>
+template <bool FULL, bool MX, typename T, typename CI, int U, int D, class F>
 __device__ __forceinline__ bool oc_pass(const RingView<T, CI>& v, RingState& r, const T* ps, int w0,
                                         unsigned rows, const T* pg, F&& f) {
   using Sh = RingShape<T, CI, U, D, 1>;
@@ -161,20 +182,20 @@ __device__ __forceinline__ bool oc_pass(const RingView<T, CI>& v, RingState& r, 
       const unsigned char* slot = v.base + r.rd * Sh::SLOT;
       r.phase ^= 1u << r.rd;
       r.rd = r.rd + 1 == D ? 0 : r.rd + 1;
-      oc_slot_of<U, FULL>(min(w, U), reinterpret_cast<const T*>(slot) + lane,
+      oc_slot_of<U, FULL, MX>(min(w, U), reinterpret_cast<const T*>(slot) + lane,
                           reinterpret_cast<const CI*>(slot + Sh::VB) + lane, ps + l, pg + w0 + l, l,
                           rows, sum);
       __syncwarp();
       ring_issue<T, CI, U, D, 1>(v, r);
       w -= U;
     } while (w > 0);
-    f(i, at, sum);
+    f(i, at, !MX || lane < (h.z >> 24), sum);
   }
   return true;
 }
 
-template <typename T, typename CI, int NW, int U, int D>
-__global__ void __launch_bounds__(NW * 32, 1) batch_onchip(const __grid_constant__ OnchipArgs a) {
+template <typename T, typename CI, int NW, int U, int D, bool MX>
+__global__ void __launch_bounds__(NW * 32, 1) onchip_groups(const __grid_constant__ OnchipArgs a) {
   using Shape = RingShape<T, CI, U, D, 1>;
   using Tm = typename std::conditional<sizeof(T) == 4, Tmem32, Tmem64>::type;
   constexpr int NT = NW * 32;
@@ -213,6 +234,9 @@ __global__ void __launch_bounds__(NW * 32, 1) batch_onchip(const __grid_constant
     uint32_t t = tm;
     for (int j = warp; j < me.nitems; j += NW, t += CS) body(items[j], items[j].y + lane, t);
   };
+  // Whether the lane's row of a slice exists (the batch's rows are padded to whole
+  // slices, a matrix's ranks are not).
+  auto exists = [&](const int4& h) { return !MX || lane < (h.z >> 24); };
   // The group's syncs, numbered in order; two arrays of partials in turn (a sum
   // may follow another without a barrier between).
   unsigned int epoch = 0;
@@ -232,14 +256,16 @@ __global__ void __launch_bounds__(NW * 32, 1) batch_onchip(const __grid_constant
                                  a.limit_ns, gs);
   };
 
-  // The window's rows of the group's other CTAs (16 bytes a load; both parts are
-  // whole slices).
+  // The window's rows of the group's other CTAs, 16 bytes a load (up to 3 of the
+  // CTA's own rows at either end come along: the group has them in L2 as well).
   auto load_window = [&]() {
     if (me.size == 1) return;
     constexpr int V = 16 / int(sizeof(T));
-    const int before = me.g0 - w0, own = 32 * me.nitems, rest = me.wrows - own;
-    for (int i = V * tid; i < rest; i += V * NT) {
-      const int l = i < before ? i : i + own;
+    const int before = (me.g0 - w0 + V - 1) / V * V, after = (me.g0 - w0 + me.rows) / V * V;
+    const int n = before + me.wrows - after;
+#pragma unroll 4
+    for (int i = V * tid; i < n; i += V * NT) {
+      const int l = i < before ? i : i - before + after;
       *reinterpret_cast<int4*>(ps + l) = __ldcg(reinterpret_cast<const int4*>(pg + w0 + l));
     }
     named_sync(1, NT);
@@ -249,16 +275,22 @@ __global__ void __launch_bounds__(NW * 32, 1) batch_onchip(const __grid_constant
   double tot[4], rr = 0.0;
   {
     double in[4] = {0.0, 0.0, 0.0, 0.0};
-    each_item([&](const int4&, int g, uint32_t t) {
-      const int pr = a.perm[me.perm0 + g];
+    each_item([&](const int4& h, int g, uint32_t t) {
       double bi = 0.0;
-      if (pr >= 0)
-        bi = me.col < 0 ? a.b_user[me.sys][pr] : a.B_user[int64_t(pr) * a.nrhs + me.col];
+      if (MX) {
+        if (exists(h)) bi = a.b[g];
+      } else {
+        const int pr = a.perm[me.perm0 + g];
+        if (pr >= 0)
+          bi = me.col < 0 ? a.b_user[me.sys][pr] : a.B_user[int64_t(pr) * a.nrhs + me.col];
+        a.b[me.vec0 + g] = bi;
+      }
       const T ri = T(bi);
-      a.b[me.vec0 + g] = bi;
-      __stcg(a.x + me.vec0 + g, 0.0);
-      ps[g - w0] = ri;
-      if (me.size > 1) __stcg(pg + g, ri);
+      if (exists(h)) {
+        __stcg(a.x + me.vec0 + g, 0.0);
+        ps[g - w0] = ri;
+        if (me.size > 1) __stcg(pg + g, ri);
+      }
       in[0] += bi * bi;
       rr += double(ri) * double(ri);
       __syncwarp();
@@ -271,7 +303,7 @@ __global__ void __launch_bounds__(NW * 32, 1) batch_onchip(const __grid_constant
     rr_part[tid] = rr;
     // Every unit has read its right-hand side before any unit's solution is
     // written (the caller may pass one buffer as both).
-    const bool all = coop_grid_barrier<NT>(a.bars, gridDim.x, a.err, a.limit_ns, gs);
+    const bool all = MX || coop_grid_barrier<NT>(a.bars, gridDim.x, a.err, a.limit_ns, gs);
     const bool ok = all && group_sum(in, tot);
     if (tid == 0) {
       sv = OcScalars{};
@@ -293,21 +325,23 @@ __global__ void __launch_bounds__(NW * 32, 1) batch_onchip(const __grid_constant
       double in[4] = {0.0, 0.0, 0.0, rr_part[tid]};
       load_window();
       const unsigned rows = unsigned(me.wrows);
-      auto row_sums = [&](int i, int at, T y) {
+      auto row_sums = [&](int i, int at, bool row, T y) {
         const uint32_t t = tm + i * CS;
         Tm rv;
         __syncwarp();
         tmem_ld(t, rv);
         tmem_st(t + C, y);
         tmem_wait_ld();
-        const double yd = double(y);
-        in[0] += double(ps[at]) * yd;
-        in[1] += double(rv.get()) * yd;
-        in[2] += yd * yd;
+        if (row) {
+          const double yd = double(y);
+          in[0] += double(ps[at]) * yd;
+          in[1] += double(rv.get()) * yd;
+          in[2] += yd * yd;
+        }
       };
       if (!(me.full
-                ? oc_pass<true, T, CI, U, D>(view(), ring, ps, w0, rows, pg, row_sums)
-                : oc_pass<false, T, CI, U, D>(view(), ring, ps, w0, rows, pg, row_sums)))
+                ? oc_pass<true, MX, T, CI, U, D>(view(), ring, ps, w0, rows, pg, row_sums)
+                : oc_pass<false, MX, T, CI, U, D>(view(), ring, ps, w0, rows, pg, row_sums)))
         if (lane == 0) atomicExch(a.err, 1);
       __syncwarp();
       tmem_wait_st();
@@ -324,8 +358,8 @@ __global__ void __launch_bounds__(NW * 32, 1) batch_onchip(const __grid_constant
       uint32_t t = tm;
       for (int j = warp; j < n; j += 2 * NW, t += 2 * CS) {
         const bool two = j + NW < n;
-        const int l0 = items[j].y - w0 + lane;
-        const int l1 = two ? items[j + NW].y - w0 + lane : l0;
+        const int4 h0 = items[j], h1 = items[two ? j + NW : j];
+        const int l0 = h0.y - w0 + lane, l1 = h1.y - w0 + lane;
         const T p0 = ps[l0], p1 = ps[l1];
         Tm r0, y0, d0, r1, y1, d1;
         __syncwarp();
@@ -341,16 +375,20 @@ __global__ void __launch_bounds__(NW * 32, 1) batch_onchip(const __grid_constant
         const T rn0 = r0.get() - alpha * y0.get(), pn0 = rn0 + beta * p0;
         tmem_st(t, rn0);
         tmem_st(t + 2 * C, d0.get() + alpha * p0);
-        ps[l0] = pn0;
-        if (me.size > 1) __stcg(pg + w0 + l0, pn0);
+        if (exists(h0)) {
+          ps[l0] = pn0;
+          if (me.size > 1) __stcg(pg + w0 + l0, pn0);
+        }
         rr += double(rn0) * double(rn0);
         if (two) {
           const T rn1 = r1.get() - alpha * y1.get(), pn1 = rn1 + beta * p1;
           __syncwarp();
           tmem_st(t + CS, rn1);
           tmem_st(t + CS + 2 * C, d1.get() + alpha * p1);
-          ps[l1] = pn1;
-          if (me.size > 1) __stcg(pg + w0 + l1, pn1);
+          if (exists(h1)) {
+            ps[l1] = pn1;
+            if (me.size > 1) __stcg(pg + w0 + l1, pn1);
+          }
           rr += double(rn1) * double(rn1);
         }
       }
@@ -361,13 +399,13 @@ __global__ void __launch_bounds__(NW * 32, 1) batch_onchip(const __grid_constant
       continue;
     }
     // R: x += d, d = 0.
-    each_item([&](const int4&, int g, uint32_t t) {
+    each_item([&](const int4& h, int g, uint32_t t) {
       Tm dv;
       __syncwarp();
       tmem_ld(t + 2 * C, dv);
       tmem_wait_ld();
       double* const xp = a.x + me.vec0 + g;
-      __stcg(xp, __ldcg(xp) + double(dv.get()));
+      if (exists(h)) __stcg(xp, __ldcg(xp) + double(dv.get()));
       __syncwarp();
       tmem_st(t + 2 * C, T(0));
     });
@@ -391,19 +429,20 @@ __global__ void __launch_bounds__(NW * 32, 1) batch_onchip(const __grid_constant
             const int64_t at = e + 32 * int64_t(in_row ? k + u : k);
             const int ci = int(idx[at]);
             v[u] = in_row ? a.vals64[at] : 0.0;
-            xv[u] = __ldcg(xu + (sizeof(CI) == 2 ? g + ci : ci));
+            xv[u] = 0.0;
+            if (!MX || !oc_padding<CI>(ci)) xv[u] = __ldcg(xu + (sizeof(CI) == 2 ? g + ci : ci));
           }
 #pragma unroll
           for (int u = 0; u < 4; ++u)
             if (k + u < w) acc += v[u] * xv[u];
         }
-        const double r64 = a.b[me.vec0 + g] - acc;
+        const double r64 = exists(h) ? a.b[me.vec0 + g] - acc : 0.0;
         const T rn = T(r64);
         Tm rv;
         __syncwarp();
         tmem_ld(t, rv);
         tmem_wait_ld();
-        const T q = ps[g - w0] - rv.get();
+        const T q = exists(h) ? ps[g - w0] - rv.get() : T(0);
         __syncwarp();
         tmem_st(t, rn);
         tmem_st(t + C, q);
@@ -421,28 +460,33 @@ __global__ void __launch_bounds__(NW * 32, 1) batch_onchip(const __grid_constant
     if (!sv.go) break;
     {
       const T s = T(sv.s), c = T(sv.c);
-      each_item([&](const int4&, int g, uint32_t t) {
+      each_item([&](const int4& h, int g, uint32_t t) {
         Tm rv, qv;
         __syncwarp();
         tmem_ld(t, rv);
         tmem_ld(t + C, qv);
         tmem_wait_ld();
         const T pn = rv.get() + s * (qv.get() - c * rv.get());
-        ps[g - w0] = pn;
-        if (me.size > 1) __stcg(pg + g, pn);
+        if (exists(h)) {
+          ps[g - w0] = pn;
+          if (me.size > 1) __stcg(pg + g, pn);
+        }
+        __syncwarp();
       });
     }
     if (!(ok = group_barrier())) break;
   }
   if (ok) {
-    each_item([&](const int4&, int g, uint32_t t) {
+    each_item([&](const int4& h, int g, uint32_t t) {
       Tm dv;
       __syncwarp();
       tmem_ld(t + 2 * C, dv);
       tmem_wait_ld();
-      const int pr = a.perm[me.perm0 + g];
-      const double xi = __ldcg(a.x + me.vec0 + g) + double(dv.get());
-      if (pr >= 0) {
+      const int pr = MX ? -1 : a.perm[me.perm0 + g];
+      const double xi = exists(h) ? __ldcg(a.x + me.vec0 + g) + double(dv.get()) : 0.0;
+      if (MX) {
+        if (exists(h)) a.x[g] = xi;
+      } else if (pr >= 0) {
         if (me.col < 0)
           a.x_user[me.sys][pr] = xi;
         else
@@ -469,14 +513,42 @@ __global__ void __launch_bounds__(NW * 32, 1) batch_onchip(const __grid_constant
   if (warp == 0) tmem_free(tm_base, uint32_t(a.alloc));
 }
 
+// Smallest and largest column of each slice of a matrix (its first row, where it
+// has no entry).
+template <typename CI>
+__global__ void __launch_bounds__(256) oc_bounds(const int4* __restrict__ items, int n,
+                                                 const CI* __restrict__ idx,
+                                                 int2* __restrict__ out) {
+  const int i = int((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = int(threadIdx.x) & 31;
+  if (i >= n) return;
+  const int4 h = items[i];
+  const int w = h.z & RING_MAX_COLS;
+  int lo = h.y, hi = h.y;
+  for (int k = 0; k < w; ++k) {
+    const int c = int(idx[(int64_t(h.x) + k) * 32 + lane]);
+    if (oc_padding<CI>(c)) continue;
+    const int col = sizeof(CI) == 2 ? h.y + lane + c : c;
+    lo = min(lo, col);
+    hi = max(hi, col);
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (lane == 0) out[i] = make_int2(lo, hi);
+}
+
 struct OcKernel {
   const void* fn;
   int64_t ring_bytes;
 };
 template <typename T, typename CI>
 OcKernel oc_kernel() {
-  return {(const void*)batch_onchip<T, CI, OC_NW, OC_U, OC_D>,
+  return {(const void*)onchip_groups<T, CI, OC_NW, OC_U, OC_D, false>,
           OC_NW * int64_t(RingShape<T, CI, OC_U, OC_D, 1>::BYTES)};
+}
+template <typename CI>
+OcKernel ocm_kernel() {
+  return {(const void*)onchip_groups<float, CI, OCM_NW, OCM_U, OCM_D, true>,
+          OCM_NW * int64_t(RingShape<float, CI, OCM_U, OCM_D, 1>::BYTES)};
 }
 OcKernel oc_kernel(bool fp32, bool d16) {
   if (fp32) return d16 ? oc_kernel<float, int16_t>() : oc_kernel<float, int32_t>();
@@ -494,7 +566,95 @@ double oc_cost(int64_t slices, double width, int64_t c) {
   return us * std::pow(double(slices), 0.2);
 }
 
+// Windows that do not fit in `fit` rows are cut down to the CTA's own rows;
+// returns the rows of the largest.
+int64_t fit_windows(OnchipPlan& p, int64_t fit) {
+  int64_t rows = 0;
+  for (OnchipCta& c : p.ctas) {
+    c.full = c.wrows <= fit;
+    if (!c.full) {
+      c.wrows = (c.rows + c.g0 - c.g0 / 4 * 4 + 3) / 4 * 4;
+      c.w0 = c.g0 / 4 * 4;
+    }
+    rows = std::max<int64_t>(rows, c.wrows);
+  }
+  return rows;
+}
+
 }  // namespace
+
+bool plan_onchip_matrix(spmv_matrix A, OnchipPlan& out) {
+  out = OnchipPlan{};
+  const bool d16 = A->fwd.d16;
+  const OcKernel kn = d16 ? ocm_kernel<int16_t>() : ocm_kernel<int32_t>();
+  out.fn = kn.fn;
+  out.block = OCM_NW * 32;
+  const ItemTable& t = item_table(A, 1);
+  if (!t.ok) return false;
+  const spmv_comm comm = A->comm;
+  const int n = t.nitems, grid = std::max(1, std::min(comm->num_sms, n));
+  std::vector<int2> bound;
+  bound.resize(size_t(n));
+  DevBuf db;
+  db.reserve(sizeof(int2) * size_t(n));
+  const int blocks = (n + 7) / 8;
+  if (d16)
+    oc_bounds<int16_t><<<blocks, 256, 0, comm->stream>>>(
+        t.desc.as<int4>(), n, A->fwd.sell_d16_global.as<int16_t>(), db.as<int2>());
+  else
+    oc_bounds<int32_t><<<blocks, 256, 0, comm->stream>>>(
+        t.desc.as<int4>(), n, A->fwd.sell_cols_global.as<int32_t>(), db.as<int2>());
+  SPMVB_CUDA(cudaGetLastError());
+  SPMVB_CUDA(cudaMemcpyAsync(bound.data(), db.ptr, sizeof(int2) * size_t(n),
+                             cudaMemcpyDeviceToHost, comm->stream));
+  SPMVB_CUDA(cudaStreamSynchronize(comm->stream));
+  int64_t most = 0, own = 0;
+  for (int b = 0; b < grid; ++b) {
+    const int a0 = int(int64_t(n) * b / grid), a1 = int(int64_t(n) * (b + 1) / grid);
+    OnchipCta c{};
+    c.item0 = a0;
+    c.nitems = a1 - a0;
+    c.g0 = t.row[size_t(a0)];
+    c.rows = t.row[size_t(a1)] - c.g0;
+    int lo = c.g0, hi = c.g0 + c.rows;
+    for (int k = a0; k < a1; ++k) {
+      lo = std::min(lo, bound[size_t(k)].x);
+      hi = std::max(hi, bound[size_t(k)].y + 1);
+    }
+    c.w0 = lo / 4 * 4;
+    c.wrows = (hi - c.w0 + 3) / 4 * 4;
+    c.bar = 0;
+    c.rank = b;
+    c.size = grid;
+    out.ctas.push_back(c);
+    most = std::max<int64_t>(most, a1 - a0);
+    own = std::max<int64_t>(own, c.rows + 8);
+  }
+  out.parts = 8 * int64_t(grid);
+  out.per_warp = int((most + OCM_NW - 1) / OCM_NW);
+  const int cols = out.per_warp * (OCM_NW / 4) * 3;
+  if (cols > 512) return false;
+  out.alloc = 32;
+  while (out.alloc < cols) out.alloc *= 2;
+  int optin = 0;
+  SPMVB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin,
+                                    comm->device));
+  cudaFuncAttributes fa{};
+  SPMVB_CUDA(cudaFuncGetAttributes(&fa, kn.fn));
+  // (32 rows more: lanes without a row read past the last one.)
+  const int64_t fixed = kn.ring_bytes + int64_t(out.per_warp) * OCM_NW * int64_t(sizeof(int4)) +
+                        32 * int64_t(sizeof(float));
+  const int64_t most_smem = optin - int64_t(fa.sharedSizeBytes);
+  if (fixed + 4 * own > most_smem) return false;
+  out.smem = fixed + 4 * fit_windows(out, (most_smem - fixed) / 4);
+  SPMVB_CUDA(cudaFuncSetAttribute(kn.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(most_smem)));
+  int nb = 0;
+  SPMVB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kn.fn, out.block,
+                                                           size_t(out.smem)));
+  out.ok = nb >= 1;
+  return out.ok;
+}
 
 bool plan_onchip(const Plan& P, int block_sys, int nrhs, bool fp32, int device, int num_sms,
                  OnchipPlan& out) {
@@ -502,6 +662,7 @@ bool plan_onchip(const Plan& P, int block_sys, int nrhs, bool fp32, int device, 
   const OcKernel kn = oc_kernel(fp32, P.fits16);
   out = OnchipPlan{};
   out.fn = kn.fn;
+  out.block = OC_NW * 32;
   if (P.entries / 32 > int64_t(INT32_MAX) || P.max_width > RING_MAX_COLS) return false;
   struct U {
     int sys, col, ctas;
@@ -575,6 +736,7 @@ bool plan_onchip(const Plan& P, int block_sys, int nrhs, bool fp32, int device, 
       c.item0 = s0 + a0;
       c.nitems = int(a1 - a0);
       c.g0 = int(32 * a0);
+      c.rows = int(32 * (a1 - a0));
       int lo = int(32 * a0), hi = int(32 * a1);
       for (int64_t k = s0 + a0; k < s0 + a1; ++k) {
         lo = std::min(lo, P.sbound[size_t(2 * k)] & ~31);
@@ -604,22 +766,7 @@ bool plan_onchip(const Plan& P, int block_sys, int nrhs, bool fp32, int device, 
   out.per_warp = int((most + OC_NW - 1) / OC_NW);
   out.alloc = 32;
   while (out.alloc < out.per_warp * (OC_NW / 4) * cols) out.alloc *= 2;
-  // Windows wider than shared memory are cut, evenly on both sides.
-  const int64_t fit = (most_smem - smem_of(out.per_warp, 0)) / vb / 32 * 32;
-  int64_t wrows = 0;
-  for (OnchipCta& c : out.ctas) {
-    c.full = c.wrows <= fit;
-    if (!c.full) {
-      const int lo = c.w0, hi = c.w0 + c.wrows, g1 = c.g0 + 32 * c.nitems;
-      const int spare = int(fit) - 32 * c.nitems;
-      int before = std::min(c.g0 - lo, spare / 64 * 32);
-      const int after = std::min(hi - g1, spare - before);
-      before = std::min(c.g0 - lo, spare - after);
-      c.w0 = c.g0 - before;
-      c.wrows = before + 32 * c.nitems + after;
-    }
-    wrows = std::max<int64_t>(wrows, c.wrows);
-  }
+  const int64_t wrows = fit_windows(out, (most_smem - smem_of(out.per_warp, 0)) / vb);
   out.smem = smem_of(out.per_warp, wrows);
   SPMVB_CUDA(cudaFuncSetAttribute(kn.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   int(most_smem)));
@@ -633,7 +780,7 @@ bool plan_onchip(const Plan& P, int block_sys, int nrhs, bool fp32, int device, 
 bool launch_onchip(const OnchipPlan& plan, OnchipArgs& a, cudaStream_t s) {
   void* args[] = {&a};
   const cudaError_t e =
-      cudaLaunchCooperativeKernel(plan.fn, dim3(unsigned(plan.ctas.size())), dim3(OC_NW * 32),
+      cudaLaunchCooperativeKernel(plan.fn, dim3(unsigned(plan.ctas.size())), dim3(unsigned(plan.block)),
                                   args, size_t(plan.smem), s);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
     (void)cudaGetLastError();

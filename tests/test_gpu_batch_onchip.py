@@ -1,4 +1,4 @@
-"""Batched solves with every unit in its own group of CTAs (batch_onchip.cu):
+"""Batched solves with every unit in its own group of CTAs (onchip.cu):
 sizes around the edges of slices, CTAs and groups, blocks of columns, both
 precisions and index widths, against the lockstep kernel on the same batch and
 the FP64 residual of the user's own matrix."""
