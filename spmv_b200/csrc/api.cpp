@@ -555,6 +555,7 @@ int spmv_comm_create(int device, void* stream, int size, spmv_comm* out) {
       require(device < count, "spmv: invalid device");
       DeviceGuard dg(device);
       SPMVB_CUDA(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device));
+      SPMVB_CUDA(cudaDeviceGetAttribute(&c->l2_bytes, cudaDevAttrL2CacheSize, device));
       if (stream) {
         c->stream.set(static_cast<cudaStream_t>(stream));
       } else {

@@ -353,11 +353,8 @@ bool run_onchip(spmv_batch B, spmv_batch_precision prec, const SolveIo& io, int 
   a.nrhs = nrhs;
   a.per_warp = p.per_warp;
   a.alloc = p.alloc;
-  // Half of L2 (24 systems of 22,000 rows, 46 MB: 13.1 us per iteration kept,
-  // 15.1 streamed; larger batches would push each other and p out).
-  int l2 = 0;
-  SPMVB_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, comm->device));
-  a.keep = B->plan.entries * int64_t((fp32 ? 4 : 8) + (B->plan.fits16 ? 2 : 4)) <= l2 / 2;
+  // (24 systems of 22,000 rows, 46 MB: 13.1 us per iteration kept, 15.1 streamed.)
+  a.keep = l2_keeps(comm, B->plan.entries * ((fp32 ? 4 : 8) + (B->plan.fits16 ? 2 : 4)));
   return launch_onchip(p, a, s);
 }
 

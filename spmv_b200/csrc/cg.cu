@@ -682,13 +682,17 @@ __global__ void __launch_bounds__(NW * 32, 1)
   __shared__ FusedScalars sv;
   __shared__ FusedCta me;
   __shared__ uint32_t tm_base;
+  __shared__ uint64_t policy;
   // Each lane's share of r.r from the update to the next product's sums.
   __shared__ double rr_part[NT];
   const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
   // Dynamic shared memory: the warps' slots, the CTA's item table, its p.
   int4* const items = reinterpret_cast<int4*>(staged_smem + NW * Shape::BYTES);
   double* const ps = reinterpret_cast<double*>(items + o.per_warp * NW);
-  if (tid == 0) me = ctas[blockIdx.x];
+  if (tid == 0) {
+    me = ctas[blockIdx.x];
+    policy = o.keep ? l2_policy_keep() : l2_policy_stream();
+  }
   if (lane == 0) ring_init<D>(bars + warp * D);
   if (warp == 0) tmem_alloc(&tm_base, uint32_t(o.alloc));
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -702,7 +706,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
                       uint32_t((warp >> 2) * o.per_warp * S * o.cols);
   auto view = [&]() {
     return RingView<double, CI>{o.vals, static_cast<const CI*>(o.idx), items, me.t1 - me.t0, NW,
-                                staged_smem + warp * Shape::BYTES, bars + warp * D};
+                                staged_smem + warp * Shape::BYTES, bars + warp * D, &policy};
   };
   RingState ring;
   ring_prime<double, CI, U, D, S>(view(), ring);
@@ -1160,6 +1164,7 @@ bool plan_onchip(spmv_matrix A, FusedPlan& plan) {
     o.vals = A->fwd.sell_vals.as<double>();
     o.idx = A->fwd.d16 ? A->fwd.sell_d16_global.ptr : A->fwd.sell_cols_global.ptr;
     o.items = t.desc.as<int4>();
+    o.keep = l2_keeps(comm, A->fwd.sz_total * (8 + (A->fwd.d16 ? 2 : 4)));
     const int64_t per_warp = (items + kn.warps - 1) / kn.warps;
     for (int cols : {6, 4})
       if (o.cols == 0 && per_warp * (kn.warps / 4) * kn.slices * cols <= 512) o.cols = cols;

@@ -168,6 +168,7 @@ struct spmv_comm_s {
   spmvb::WorkStream stream;
   bool own_stream = false;
   int num_sms = 0;
+  int l2_bytes = 0;
   // References: the caller's handle plus one per live map or matrix, so the
   // communicator outlives everything created on it, whatever the order of
   // the destroy calls.
@@ -373,6 +374,9 @@ spmv_kernel pick_kernel(spmv_kernel requested, const DevCsr& C, bool allow_sell 
 // Lanes per row picked from the mean row length (vector kernel).
 int auto_width(double mean_row, spmv_dtype dtype);
 int max_blocks_for(int num_sms, int BS);
+// Whether a matrix streamed once per iteration should be kept in L2: half of it
+// (larger ones push p and x out without staying themselves).
+bool l2_keeps(spmv_comm comm, int64_t bytes);
 // SELL-32 layout (sell.cu): built on the device from the device CSR.
 int64_t sell_padded_size(const std::vector<int32_t>& rowptr, int32_t nrows,
                          std::vector<int32_t>* soff);
@@ -458,6 +462,7 @@ struct OnchipShape {
   int per_warp = 0;               // items per warp at most
   int cols = 0;                   // tensor memory columns per slice: r, y (4) and x (6)
   int alloc = 0;                  // columns allocated per CTA
+  bool keep = false;              // L2 should hold the entries (l2_keeps)
 };
 struct FusedPlan {
   const void* fn = nullptr;

@@ -207,11 +207,15 @@ __global__ void __launch_bounds__(NW * 32, 1) onchip_groups(const __grid_constan
   __shared__ OcScalars sv;
   __shared__ OnchipCta me;
   __shared__ uint32_t tm_base;
+  __shared__ uint64_t policy;
   __shared__ double rr_part[NT];
   const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
   int4* const items = reinterpret_cast<int4*>(oc_smem + NW * Shape::BYTES);
   T* const ps = reinterpret_cast<T*>(items + a.per_warp * NW);
-  if (tid == 0) me = a.ctas[blockIdx.x];
+  if (tid == 0) {
+    me = a.ctas[blockIdx.x];
+    policy = a.keep ? l2_policy_keep() : l2_policy_stream();
+  }
   if (lane == 0) ring_init<D>(bars + warp * D);
   if (warp == 0) tmem_alloc(&tm_base, uint32_t(a.alloc));
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -224,7 +228,7 @@ __global__ void __launch_bounds__(NW * 32, 1) onchip_groups(const __grid_constan
   auto view = [&]() {
     return RingView<T, CI>{static_cast<const T*>(a.vals), static_cast<const CI*>(a.idx), items,
                            me.nitems, NW, oc_smem + warp * Shape::BYTES, bars + warp * D,
-                           a.keep};
+                           &policy};
   };
   RingState ring;
   ring_prime<T, CI, U, D, 1>(view(), ring);

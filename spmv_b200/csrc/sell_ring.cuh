@@ -44,7 +44,7 @@ struct RingView {
   int count, stride;    // items of the CTA; the warp takes warp, warp + stride, ...
   unsigned char* base;  // the warp's slots
   uint64_t* bar;        // and their barriers
-  bool keep = false;    // L2 should hold the entries from one pass to the next
+  const uint64_t* policy;  // the copies' L2 policy (shared memory)
 };
 
 // State of a warp's ring (registers).
@@ -76,7 +76,7 @@ __device__ __forceinline__ void ring_issue(const RingView<T, CI>& v, RingState& 
     uint64_t* bar = v.bar + r.fill;
     mbar_arrive_expect_tx(bar, n * uint32_t(sizeof(T) + sizeof(CI)));
     if (n > 0) {
-      const uint64_t policy = v.keep ? l2_policy_keep() : l2_policy_stream();
+      const uint64_t policy = *v.policy;
       bulk_g2s(s, v.vals + e, n * uint32_t(sizeof(T)), bar, policy);
       bulk_g2s(s + Sh::VB, v.idx + e, n * uint32_t(sizeof(CI)), bar, policy);
     }

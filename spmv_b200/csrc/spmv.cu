@@ -271,6 +271,8 @@ spmv_kernel pick_kernel(spmv_kernel requested, const DevCsr& C, bool allow_sell)
   return SPMV_KERNEL_VECTOR;
 }
 
+bool l2_keeps(spmv_comm comm, int64_t bytes) { return bytes <= comm->l2_bytes / 2; }
+
 int max_blocks_for(int num_sms, int BS) {
   // One wave of resident CTAs (2048 threads per SM), times two so that a
   // CTA finishing early finds work without waiting for the tail.
