@@ -354,7 +354,7 @@ bool run_onchip(spmv_batch B, spmv_batch_precision prec, const SolveIo& io, int 
   a.per_warp = p.per_warp;
   a.alloc = p.alloc;
   // (24 systems of 22,000 rows, 46 MB: 13.1 us per iteration kept, 15.1 streamed.)
-  a.keep = l2_keeps(comm, B->plan.entries * ((fp32 ? 4 : 8) + (B->plan.fits16 ? 2 : 4)));
+  a.keep = l2_share(comm, B->plan.entries * ((fp32 ? 4 : 8) + (B->plan.fits16 ? 2 : 4)));
   return launch_onchip(p, a, s);
 }
 

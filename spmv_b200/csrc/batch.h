@@ -198,7 +198,7 @@ struct OnchipArgs {
   unsigned long long limit_ns;
   double rtol2, delta2;
   int kmax, nrhs, per_warp, alloc;
-  bool keep;  // the matrices fit in L2 with room to spare
+  float keep;  // share of the matrices L2 should hold (l2_share)
 };
 
 // Groups of CTAs for the batch's systems (and nrhs columns of block_sys); false

@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
   double* const ps = reinterpret_cast<double*>(items + o.per_warp * NW);
   if (tid == 0) {
     me = ctas[blockIdx.x];
-    policy = o.keep ? l2_policy_keep() : l2_policy_stream();
+    policy = o.keep > 0.0f ? l2_policy_part(o.keep) : l2_policy_stream();
   }
   if (lane == 0) ring_init<D>(bars + warp * D);
   if (warp == 0) tmem_alloc(&tm_base, uint32_t(o.alloc));
@@ -1164,11 +1164,13 @@ bool plan_onchip(spmv_matrix A, FusedPlan& plan) {
     o.vals = A->fwd.sell_vals.as<double>();
     o.idx = A->fwd.d16 ? A->fwd.sell_d16_global.ptr : A->fwd.sell_cols_global.ptr;
     o.items = t.desc.as<int4>();
-    o.keep = l2_keeps(comm, A->fwd.sz_total * (8 + (A->fwd.d16 ? 2 : 4)));
     const int64_t per_warp = (items + kn.warps - 1) / kn.warps;
     for (int cols : {6, 4})
       if (o.cols == 0 && per_warp * (kn.warps / 4) * kn.slices * cols <= 512) o.cols = cols;
     if (o.cols == 0) continue;
+    // (With x in global memory its traffic needs that room: 7-point 128^3 36.7 us
+    // per iteration streamed, 41.3 with half of L2 kept; 5-point 1400^2 26.2, 30.8.)
+    if (o.cols == 6) o.keep = l2_share(comm, A->fwd.sz_total * (8 + (A->fwd.d16 ? 2 : 4)));
     o.per_warp = int(per_warp);
     o.alloc = 32;
     while (o.alloc < per_warp * (kn.warps / 4) * kn.slices * o.cols) o.alloc *= 2;

@@ -374,9 +374,12 @@ spmv_kernel pick_kernel(spmv_kernel requested, const DevCsr& C, bool allow_sell 
 // Lanes per row picked from the mean row length (vector kernel).
 int auto_width(double mean_row, spmv_dtype dtype);
 int max_blocks_for(int num_sms, int BS);
-// Whether a matrix streamed once per iteration should be kept in L2: half of it
-// (larger ones push p and x out without staying themselves).
-bool l2_keeps(spmv_comm comm, int64_t bytes);
+// The share of a matrix, streamed once per iteration by a solver whose vectors are
+// on chip, that L2 should hold from one iteration to the next (the same lines each
+// time): as much as half of it holds.  us per iteration by the part of L2 kept, 0 /
+// 0.3 / 0.5 / 0.85: mixed 27-point 96^3 (149 MB) 30.9 / 28.0 / 28.1 / 32.2; 7-point
+// 112^3 (98 MB) 25.7 / 24.5 / 24.2 / 26.1; 5-point 1024^2 (52 MB) 14.8 / 14.0 / 14.0 / 13.9.
+float l2_share(spmv_comm comm, int64_t bytes);
 // SELL-32 layout (sell.cu): built on the device from the device CSR.
 int64_t sell_padded_size(const std::vector<int32_t>& rowptr, int32_t nrows,
                          std::vector<int32_t>* soff);
@@ -462,7 +465,7 @@ struct OnchipShape {
   int per_warp = 0;               // items per warp at most
   int cols = 0;                   // tensor memory columns per slice: r, y (4) and x (6)
   int alloc = 0;                  // columns allocated per CTA
-  bool keep = false;              // L2 should hold the entries (l2_keeps)
+  float keep = 0.0f;              // share of the entries L2 should hold (l2_share)
 };
 struct FusedPlan {
   const void* fn = nullptr;

@@ -1014,7 +1014,7 @@ bool ir_use_onchip(spmv_matrix A, IrWorkspace& w) {
   a.b = w.b.as<double>();
   a.per_warp = p.per_warp;
   a.alloc = p.alloc;
-  a.keep = l2_keeps(A->comm, C.sz_total * (4 + (C.d16 ? 2 : 4)));
+  a.keep = l2_share(A->comm, C.sz_total * (4 + (C.d16 ? 2 : 4)));
   w.oargs = a;
   return true;
 }

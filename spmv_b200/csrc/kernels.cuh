@@ -171,6 +171,14 @@ __device__ __forceinline__ uint64_t l2_policy_stream() {
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
+// `fraction` of the lines (the same ones each time) kept, the others evicted first.
+__device__ __forceinline__ uint64_t l2_policy_part(float fraction) {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, %1;"
+               : "=l"(p)
+               : "f"(fraction));
+  return p;
+}
 __device__ __forceinline__ double ld_pol(const double* a, uint64_t pol) {
   double v;
   asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(a), "l"(pol));

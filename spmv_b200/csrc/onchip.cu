@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(NW * 32, 1) onchip_groups(const __grid_constan
   T* const ps = reinterpret_cast<T*>(items + a.per_warp * NW);
   if (tid == 0) {
     me = a.ctas[blockIdx.x];
-    policy = a.keep ? l2_policy_keep() : l2_policy_stream();
+    policy = a.keep > 0.0f ? l2_policy_part(a.keep) : l2_policy_stream();
   }
   if (lane == 0) ring_init<D>(bars + warp * D);
   if (warp == 0) tmem_alloc(&tm_base, uint32_t(a.alloc));

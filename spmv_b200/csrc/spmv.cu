@@ -271,7 +271,9 @@ spmv_kernel pick_kernel(spmv_kernel requested, const DevCsr& C, bool allow_sell)
   return SPMV_KERNEL_VECTOR;
 }
 
-bool l2_keeps(spmv_comm comm, int64_t bytes) { return bytes <= comm->l2_bytes / 2; }
+float l2_share(spmv_comm comm, int64_t bytes) {
+  return float(std::min(1.0, 0.5 * comm->l2_bytes / double(std::max<int64_t>(bytes, 1))));
+}
 
 int max_blocks_for(int num_sms, int BS) {
   // One wave of resident CTAs (2048 threads per SM), times two so that a
