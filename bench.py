@@ -701,12 +701,14 @@ def run_ours(args, info):
         cg_bytes = b_iter * k_mean
         cg_ach = cg_bytes / t_launch / 1e9
         matrix_bytes = nnz * (8 + cg_bits // 8) * k_mean
+        onchip = cg_form[2].startswith("tmem")
         cg_traffic = None
         if tp.exists():
             try:
-                merged = bool(cg_form[2] and cg_form[2].endswith(":m"))
+                merged = cg_form[2].endswith(":m")
                 cg_traffic = json.loads(tp.read_text()).get(
-                    "cg_fused_merged_c2" if merged else "cg_fused_c2")
+                    "cg_onchip_c2" if onchip else "cg_fused_merged_c2" if merged
+                    else "cg_fused_c2")
             except Exception:
                 cg_traffic = None
         # achieved / frac count the compulsory DRAM bytes: the matrix stream
@@ -719,8 +721,11 @@ def run_ours(args, info):
                    "traffic_source": "profiles/traffic.json: dram__bytes_read.sum + "
                                      "dram__bytes_write.sum of one launch, committed ncu "
                                      "capture (not measured in this run)",
-                   "kernel": f"cg_fused ({cg_form[1]} CTAs/SM, r in {cg_form[2].split(':')[0]}, "
-                             f"staged width {cg_w}, {cg_bits}-bit indices, "
+                   "kernel": (f"cg_onchip (1 CTA/SM, p in shared, r and y in tensor memory, "
+                              f"per-warp rings, {cg_bits}-bit indices, " if onchip else
+                              f"cg_fused ({cg_form[1]} CTAs/SM, r in "
+                              f"{cg_form[2].split(':')[0]}, staged width {cg_w}, "
+                              f"{cg_bits}-bit indices, ") +
                              f"{2 if cg_form[2].endswith(':m') else 3} grid syncs per "
                              "iteration; one launch per solve)",
                    "bytes_per_launch": matrix_bytes, "us_per_launch": t_launch * 1e6,
