@@ -1,7 +1,7 @@
 // Batched solves: API, device layout, launch and autotuner (no counterpart
 // in the reference; the recurrences are spmv::cg's, cg.cpp:50-80, on the
-// product of Matrix::operator*, Matrix.cpp:199-204).  The kernel is
-// batch_kernel.cuh, the host planning batch_plan.cpp.
+// product of Matrix::operator*, Matrix.cpp:199-204).  The kernels are
+// onchip.cu's and batch_kernel.cuh's, the host planning is batch_plan.cpp.
 #include <algorithm>
 #include <chrono>
 #include <cmath>

@@ -1,6 +1,6 @@
 // Batched solver internals shared by the planner (batch_plan.cpp), the API
-// and autotuner (batch.cu) and the kernel instantiations (batch_f32.cu,
-// batch_f64.cu).  No counterpart in the reference: the batch builds on
+// and autotuner (batch.cu), the kernel instantiations (batch_f32.cu,
+// batch_f64.cu) and the on-chip form (onchip.cu).  No counterpart in the reference: the batch builds on
 // spmv::cg (cg.cpp:11-83) and Matrix::operator* (Matrix.cpp:199-204).
 #pragma once
 

@@ -663,9 +663,9 @@ __global__ void __launch_bounds__(CFG::BS, CFG::MINB)
 // own ring (sell_ring.cuh).
 //
 // Measured (us per iteration; the form the workspace chose before): 7-point
-// 128^3 over 8 ranks 37.4 (42.3), of which the product takes 25 (the matrix at
+// 128^3 over 8 ranks 36.7 (42.3), of which the product takes 25 (the matrix at
 // 5.8 TB/s), the sum 4, the update 6 (x and p through L2) and the barrier 1.5;
-// 96^3 18.3 (22.3); 5-point 1024^2, x in tensor memory, 14.8 (20.3), product 7.6;
+// 96^3 16.7 (22.3); 5-point 1024^2, x in tensor memory, 14.1 (20.3);
 // 48^3 and below 6.3 to 6.7 (17 to 20 as a CUDA graph): there the two syncs
 // (2.9 + 1.4) are most of it.
 template <int NW, int U, int D, int S, bool LATE, bool D16>

@@ -1154,8 +1154,8 @@ void ir_choose_form(spmv_matrix A, IrWorkspace& w) {
   }
   // Where every CTA's window of p fits, the other forms have not been faster (us
   // per inner iteration, on chip, the best other fused plan, graph: 27-point 96^3
-  // 30.5, 41.3, 51.8; 40^3 8.2, 10.7, 24.7; 7-point 64^3 8.7, 11.3, 24.8; 5-point
-  // 1024^2 14.5, 17.3, 30.5; 1400^2 22.3, 25.4, 38.6), so nothing is timed.  Where
+  // 28.1, 41.3, 51.8; 40^3 8.1, 10.7, 24.7; 7-point 64^3 8.6, 11.3, 24.8; 5-point
+  // 1024^2 14.3, 17.3, 30.5; 1400^2 22.1, 25.4, 38.6), so nothing is timed.  Where
   // one does not (7-point 128^3: 33.0, 31.2, 44.8), every plan that fits is.
   if (onchip && ir_use_onchip(A, w)) {
     bool full = true;

@@ -38,9 +38,9 @@
 // and 5 columns: 63 us in the lockstep kernel, 5.6 here; 24 of 22,000 and 32
 // columns, the chip full, 105 and 24.
 // One matrix, mixed (the fused form of ir.cu before): 27-point 96^3 41.3 us per
-// iteration, now 30.5 (of which its entries are 22 at the rate of a copy); 5-point
-// 1024^2 17.3 and 14.5, 200 x 180 19.1 and 5.8 (as a CUDA graph before); 27-point
-// 40^3 10.7 and 8.2.
+// iteration, now 28.1 (its entries are 22 at the rate of a copy); 5-point 1024^2
+// 17.3 and 14.3, 200 x 180 19.1 and 5.8 (as a CUDA graph before); 27-point 40^3
+// 10.7 and 8.1.
 #include <algorithm>
 #include <cmath>
 #include <queue>
@@ -62,7 +62,7 @@ constexpr int OC_U = 16;
 constexpr int OC_D = 1;
 
 // The same for one matrix over the grid, whose entries come from memory: more
-// warps and copies in flight (us per iteration, 27-point 96^3 / 5-point 1024^2 /
+// warps and copies in flight (us per iteration with nothing kept in L2, 27-point 96^3 / 5-point 1024^2 /
 // 7-point 128^3: 28 warps 9 x 2 30.5 / 14.5 / 33.0; 24 warps 9 x 2 30.5 / 15.4 / 36.9;
 // 20 warps 9 x 3 30.8 / 15.7 / 40.7, 14 x 2 30.7 / 15.9 / 41.7, 16 x 1 34.5 / 18.3 / 46.2).
 constexpr int OCM_NW = 28;
