@@ -1681,9 +1681,9 @@ template <typename T, typename CI, int R>
 bool launch_one(const Args<T, CI>& a, int cps, int num_sms, cudaStream_t s, bool dry) {
   const void* fn = reinterpret_cast<const void*>(lockstep_kernel<T, CI, R>);
   const size_t smem = dyn_smem(a);
-  if (smem > 48 * 1024)
-    SPMVB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  int nb = 0;
+  int device = 0, nb = 0;
+  SPMVB_CUDA(cudaGetDevice(&device));
+  if (int64_t(smem) > allow_dynamic_smem(fn, device)) return false;
   SPMVB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, NT, smem));
   if (nb < cps) return false;
   if (dry) return true;

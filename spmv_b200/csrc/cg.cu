@@ -1421,18 +1421,24 @@ bool fused_plan(spmv_matrix A, const DevCsr::StagedTable& t, const void* fn, int
   return true;
 }
 
-bool fused_fits(spmv_comm comm, const void* fn, int block, int cps, int64_t smem,
-                FusedPlan& plan) {
+int64_t allow_dynamic_smem(const void* fn, int device) {
   int optin = 0;
-  SPMVB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin,
-                                    comm->device));
+  SPMVB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   cudaFuncAttributes fa{};
   SPMVB_CUDA(cudaFuncGetAttributes(&fa, fn));
-  if (smem + int64_t(fa.sharedSizeBytes) > optin) return false;
-  SPMVB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  const int64_t most = optin - int64_t(fa.sharedSizeBytes);
+  SPMVB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)));
+  return most;
+}
+
+bool fused_fits(spmv_comm comm, const void* fn, int block, int cps, int64_t smem,
+                FusedPlan& plan) {
+  if (smem > allow_dynamic_smem(fn, comm->device)) return false;
   int nb = 0;
   SPMVB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, block, size_t(smem)));
   if (nb < cps) {
+    cudaFuncAttributes fa{};
+    SPMVB_CUDA(cudaFuncGetAttributes(&fa, fn));
     debug_log("fused plan: " + std::to_string(nb) + " of " + std::to_string(cps) +
               " CTAs fit, registers " + std::to_string(fa.numRegs) + ", shared memory " +
               std::to_string(smem) + " + " + std::to_string(fa.sharedSizeBytes));

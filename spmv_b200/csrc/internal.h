@@ -482,6 +482,11 @@ struct FusedPlan {
 // of the longest run in shared memory; false when it does not fit.
 bool fused_plan(spmv_matrix A, const DevCsr::StagedTable& t, const void* fn, int block,
                 int cps, int64_t stage_smem, int rs_bytes, FusedPlan& plan);
+// Bytes of dynamic shared memory a CTA of `fn` can have.  Sets the kernel's limit
+// to that, whatever one launch needs: the limit belongs to the function, so one
+// matrix's smaller launch (or another thread's) must not lower it under a plan kept
+// for a larger one.
+int64_t allow_dynamic_smem(const void* fn, int device);
 // Whether `cps` CTAs of `block` threads of `fn` with `smem` bytes of dynamic
 // shared memory fit an SM; sets the plan's kernel, block and shared memory.
 bool fused_fits(spmv_comm comm, const void* fn, int block, int cps, int64_t smem,

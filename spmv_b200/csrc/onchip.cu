@@ -640,19 +640,12 @@ bool plan_onchip_matrix(spmv_matrix A, OnchipPlan& out) {
   if (cols > 512) return false;
   out.alloc = 32;
   while (out.alloc < cols) out.alloc *= 2;
-  int optin = 0;
-  SPMVB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin,
-                                    comm->device));
-  cudaFuncAttributes fa{};
-  SPMVB_CUDA(cudaFuncGetAttributes(&fa, kn.fn));
   // (32 rows more: lanes without a row read past the last one.)
   const int64_t fixed = kn.ring_bytes + int64_t(out.per_warp) * OCM_NW * int64_t(sizeof(int4)) +
                         32 * int64_t(sizeof(float));
-  const int64_t most_smem = optin - int64_t(fa.sharedSizeBytes);
+  const int64_t most_smem = allow_dynamic_smem(kn.fn, comm->device);
   if (fixed + 4 * own > most_smem) return false;
   out.smem = fixed + 4 * fit_windows(out, (most_smem - fixed) / 4);
-  SPMVB_CUDA(cudaFuncSetAttribute(kn.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  int(most_smem)));
   int nb = 0;
   SPMVB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kn.fn, out.block,
                                                            size_t(out.smem)));
@@ -687,15 +680,11 @@ bool plan_onchip(const Plan& P, int block_sys, int nrhs, bool fp32, int device, 
   for (int l = 0; l < nrhs; ++l) add(block_sys, l);
   if (units.empty() || int(units.size()) > num_sms) return false;
   // Slices a CTA can hold: tensor memory's 512 columns, shared memory.
-  int optin = 0;
-  SPMVB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-  cudaFuncAttributes fa{};
-  SPMVB_CUDA(cudaFuncGetAttributes(&fa, kn.fn));
   const int cols = 3 * vb / 4;
   auto smem_of = [&](int per_warp, int64_t rows) {
     return kn.ring_bytes + int64_t(per_warp) * OC_NW * int64_t(sizeof(int4)) + rows * vb;
   };
-  const int64_t most_smem = optin - int64_t(fa.sharedSizeBytes);
+  const int64_t most_smem = allow_dynamic_smem(kn.fn, device);
   int per_warp = 512 / (OC_NW / 4 * cols);
   while (per_warp > 0 && smem_of(per_warp, 32 * per_warp * OC_NW) > most_smem) --per_warp;
   if (per_warp == 0) return false;
@@ -772,8 +761,6 @@ bool plan_onchip(const Plan& P, int block_sys, int nrhs, bool fp32, int device, 
   while (out.alloc < out.per_warp * (OC_NW / 4) * cols) out.alloc *= 2;
   const int64_t wrows = fit_windows(out, (most_smem - smem_of(out.per_warp, 0)) / vb);
   out.smem = smem_of(out.per_warp, wrows);
-  SPMVB_CUDA(cudaFuncSetAttribute(kn.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  int(most_smem)));
   int nb = 0;
   SPMVB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kn.fn, OC_NW * 32,
                                                            size_t(out.smem)));
