@@ -780,7 +780,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
                   tmem_ld(t + q * o.cols, rv[q]);
                   tmem_st(t + q * o.cols + 2, sum[q]);
                 }
-                tmem_wait_ld();
+                tmem_wait_ld(rv);
 #pragma unroll
                 for (int q = 0; q < S; ++q) {
                   if (row.valid[q]) {
@@ -826,21 +826,26 @@ __global__ void __launch_bounds__(NW * 32, 1)
 #pragma unroll
         for (int h = 0; h < B; ++h) row[h] = RingRows<S>(items[min(j + h * NW, n - 1)]);
         __syncwarp();
+        // (Of an item that is not there the first's columns again, and r for an x
+        // that is not in tensor memory: not used.)
 #pragma unroll
         for (int h = 0; h < B; ++h)
-          if (h == 0 || j + NW < n)
 #pragma unroll
-            for (int q = 0; q < S; ++q) {
-              const uint32_t tq = t + (h * S + q) * o.cols;
-              tmem_ld(tq, rv[h][q]);
-              tmem_ld(tq + 2, yv[h][q]);
-              if (xt)
-                tmem_ld(tq + 4, xv[h][q]);
-              else if (row[h].valid[q])
-                xg[h][q] = ld_pol(c.x + row[h].g[q], keep);
-            }
+          for (int q = 0; q < S; ++q) {
+            const uint32_t tq = t + ((j + h * NW < n ? h * S : 0) + q) * o.cols;
+            tmem_ld(tq, rv[h][q]);
+            tmem_ld(tq + 2, yv[h][q]);
+            tmem_ld(tq + (xt ? 4 : 0), xv[h][q]);
+          }
+        if (!xt)
+#pragma unroll
+          for (int h = 0; h < B; ++h)
+            if (h == 0 || j + NW < n)
+#pragma unroll
+              for (int q = 0; q < S; ++q)
+                if (row[h].valid[q]) xg[h][q] = ld_pol(c.x + row[h].g[q], keep);
         __syncwarp();
-        tmem_wait_ld();
+        tmem_wait_ld(rv, yv, xv);
 #pragma unroll
         for (int h = 0; h < B; ++h)
           if (h == 0 || j + NW < n)
@@ -881,7 +886,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
         Tmem64 xv;
         __syncwarp();
         tmem_ld(t + q * o.cols + 4, xv);
-        tmem_wait_ld();
+        tmem_wait_ld(xv);
         if (row.valid[q]) c.x[row.g[q]] = xv.get();
       }
     });

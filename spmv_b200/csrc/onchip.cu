@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(NW * 32, 1) onchip_groups(const __grid_constan
         __syncwarp();
         tmem_ld(t, rv);
         tmem_st(t + C, y);
-        tmem_wait_ld();
+        tmem_wait_ld(rv);
         if (row) {
           const double yd = double(y);
           in[0] += double(ps[at]) * yd;
@@ -370,12 +370,11 @@ __global__ void __launch_bounds__(NW * 32, 1) onchip_groups(const __grid_constan
         tmem_ld(t, r0);
         tmem_ld(t + C, y0);
         tmem_ld(t + 2 * C, d0);
-        if (two) {
-          tmem_ld(t + CS, r1);
-          tmem_ld(t + CS + C, y1);
-          tmem_ld(t + CS + 2 * C, d1);
-        }
-        tmem_wait_ld();
+        const uint32_t t1 = two ? t + CS : t;  // (the first's again: not used)
+        tmem_ld(t1, r1);
+        tmem_ld(t1 + C, y1);
+        tmem_ld(t1 + 2 * C, d1);
+        tmem_wait_ld(r0, y0, d0, r1, y1, d1);
         const T rn0 = r0.get() - alpha * y0.get(), pn0 = rn0 + beta * p0;
         tmem_st(t, rn0);
         tmem_st(t + 2 * C, d0.get() + alpha * p0);
@@ -407,7 +406,7 @@ __global__ void __launch_bounds__(NW * 32, 1) onchip_groups(const __grid_constan
       Tm dv;
       __syncwarp();
       tmem_ld(t + 2 * C, dv);
-      tmem_wait_ld();
+      tmem_wait_ld(dv);
       double* const xp = a.x + me.vec0 + g;
       if (exists(h)) __stcg(xp, __ldcg(xp) + double(dv.get()));
       __syncwarp();
@@ -445,7 +444,7 @@ __global__ void __launch_bounds__(NW * 32, 1) onchip_groups(const __grid_constan
         Tm rv;
         __syncwarp();
         tmem_ld(t, rv);
-        tmem_wait_ld();
+        tmem_wait_ld(rv);
         const T q = exists(h) ? ps[g - w0] - rv.get() : T(0);
         __syncwarp();
         tmem_st(t, rn);
@@ -469,7 +468,7 @@ __global__ void __launch_bounds__(NW * 32, 1) onchip_groups(const __grid_constan
         __syncwarp();
         tmem_ld(t, rv);
         tmem_ld(t + C, qv);
-        tmem_wait_ld();
+        tmem_wait_ld(rv, qv);
         const T pn = rv.get() + s * (qv.get() - c * rv.get());
         if (exists(h)) {
           ps[g - w0] = pn;
@@ -485,7 +484,7 @@ __global__ void __launch_bounds__(NW * 32, 1) onchip_groups(const __grid_constan
       Tm dv;
       __syncwarp();
       tmem_ld(t + 2 * C, dv);
-      tmem_wait_ld();
+      tmem_wait_ld(dv);
       const int pr = MX ? -1 : a.perm[me.perm0 + g];
       const double xi = exists(h) ? __ldcg(a.x + me.vec0 + g) + double(dv.get()) : 0.0;
       if (MX) {

@@ -238,15 +238,10 @@ __device__ __forceinline__ void tmem_free(uint32_t addr, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols)
                : "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void tmem_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
-// 64-bit values in two columns.  A load's registers are valid after
-// tmem_wait_ld(), so callers wait before anything else can need a register
-// (nothing is spilled in between).
+// 64-bit values in two columns.
 struct Tmem64 {
   uint32_t lo, hi;
   __device__ __forceinline__ double get() const { return __hiloint2double(int(hi), int(lo)); }
@@ -273,6 +268,25 @@ __device__ __forceinline__ void tmem_st(uint32_t addr, float v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(addr),
                "r"(__float_as_uint(v))
                : "memory");
+}
+// A load's registers are valid after the wait.  tmem_wait_ld takes every value that
+// is in flight and gives each of them back from behind the wait, so that nothing
+// computed from one can be moved ahead of it.  The loads are unconditional, so that
+// no copy of a register is made between a load and its wait.
+__device__ __forceinline__ void tmem_landed(Tmem64& a) {
+  asm volatile("" : "+r"(a.lo), "+r"(a.hi));
+}
+__device__ __forceinline__ void tmem_landed(Tmem32& a) { asm volatile("" : "+r"(a.v)); }
+template <class R, int N>
+__device__ __forceinline__ void tmem_landed(R (&a)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) tmem_landed(a[i]);
+}
+template <class... R>
+__device__ __forceinline__ void tmem_wait_ld(R&... loaded) {
+  static_assert(sizeof...(R) > 0, "the values that the wait is for");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  (tmem_landed(loaded), ...);
 }
 
 }  // namespace spmvb
