@@ -117,8 +117,10 @@ int spmv_comm_stream(spmv_comm comm, void** stream);
  * leave = 2 and 3: the same around calls that only put work on a stream
  * (update, reverse_update, mult, transpmult, mult_block, sample_outer); when
  * `stream` is the legacy default stream (NULL) and the communicator made its
- * own stream, which spmv_comm_stream has not handed out, the calls this thread
- * makes in between put their work on `stream` itself. */
+ * own stream, which spmv_comm_stream has not handed out and no other thread's
+ * call works on, the calls this thread makes in between put their work on
+ * `stream` itself.  Calls of other threads that need the communicator's stream
+ * wait for leave = 3, so nothing but such calls belongs in between. */
 int spmv_comm_fence(spmv_comm comm, void* stream, int leave);
 int spmv_comm_synchronize(spmv_comm comm);
 

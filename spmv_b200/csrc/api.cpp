@@ -46,75 +46,6 @@ DeviceGuard::~DeviceGuard() {
 
 namespace {
 
-// One event per thread and device, made on first use: it is recorded and the
-// other stream made to wait for it at once, so a thread can use its own again
-// for the next pair.
-struct FenceEvents {
-  std::vector<cudaEvent_t> ev;  // per device
-  cudaEvent_t get(int device) {
-    if (int(ev.size()) <= device) ev.resize(size_t(device) + 1, nullptr);
-    if (!ev[size_t(device)])
-      SPMVB_CUDA(cudaEventCreateWithFlags(&ev[size_t(device)], cudaEventDisableTiming));
-    return ev[size_t(device)];
-  }
-  ~FenceEvents() {
-    for (cudaEvent_t e : ev)
-      if (e) soft_check(cudaEventDestroy(e), "cudaEventDestroy");
-  }
-};
-thread_local FenceEvents g_fence;
-// The communicator's stream whose direct fence this thread is in.
-thread_local const WorkStream* g_direct = nullptr;
-
-// Work put on `after` from here on waits for the work now on `before`.
-void order_streams(int device, cudaStream_t before, cudaStream_t after) {
-  cudaEvent_t e = g_fence.get(device);
-  SPMVB_CUDA(cudaEventRecord(e, before));
-  SPMVB_CUDA(cudaStreamWaitEvent(after, e, 0));
-}
-
-}  // namespace
-
-cudaStream_t WorkStream::get() const {
-  const std::lock_guard<std::mutex> lock(mu_);
-  if (g_direct == this) {
-    if (own_ahead_) {  // another thread's work since the fence began
-      order_streams(device_, own_, nullptr);
-      own_ahead_ = false;
-    }
-    default_ahead_ = true;
-    return nullptr;
-  }
-  if (default_ahead_) {
-    order_streams(device_, nullptr, own_);
-    default_ahead_ = false;
-  }
-  own_ahead_ = true;
-  return own_;
-}
-
-void WorkStream::hand_out() const {
-  (void)get();  // what follows on the handle is behind the direct work
-  const std::lock_guard<std::mutex> lock(mu_);
-  given_ = true;
-}
-
-bool WorkStream::begin_direct(int device) const {
-  const std::lock_guard<std::mutex> lock(mu_);
-  if (given_ || g_direct != nullptr) return false;
-  device_ = device;
-  g_direct = this;
-  return true;
-}
-
-bool WorkStream::end_direct() const {
-  if (g_direct != this) return false;
-  g_direct = nullptr;
-  return true;
-}
-
-namespace {
-
 void check_comm(spmv_comm c) { require(c != nullptr, "spmv: communicator is NULL"); }
 void check_map(spmv_l2gmap m) { require(m != nullptr, "spmv: L2GMap is NULL"); }
 void check_mat(spmv_matrix A) { require(A != nullptr, "spmv: Matrix is NULL"); }

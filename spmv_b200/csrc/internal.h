@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <condition_variable>
 #include <cstdint>
 #include <functional>
 #include <memory>
@@ -49,9 +50,17 @@ void soft_check(cudaError_t e, const char* what);
                     std::string(#call) + ": " + cudaGetErrorString(e_));     \
   } while (0)
 
+// A library call of this thread: the communicators' streams that it asks for are in
+// use until it ends (WorkStream).
+struct CallScope {
+  CallScope();
+  ~CallScope();
+};
+
 // Runs `body` and turns exceptions into a status code.
 template <class F>
 int guard(F&& body) {
+  const CallScope call;
   try {
     body();
     return SPMV_SUCCESS;
@@ -129,33 +138,45 @@ struct DeviceGuard {
 
 namespace spmvb {
 
-// The stream a communicator's work goes to, asked for at each use.
+// The stream a communicator's work goes to, asked for at each use (stream.cpp).
 //
 // That is `own`, except while the calling thread is inside a direct fence
 // (spmv_comm_fence, leave = 2 and 3): then it is the legacy default stream, the
 // one the caller's vectors are ordered on, and a call costs no wait between
 // two streams (four per ghost update and product: about 9 us of a 42 us pass).
 // Direct fences are for a stream the library made and has not handed out, so
-// that nobody else puts work on it; uses of the two streams are joined by an
-// event where one follows the other, whichever thread makes them.
+// that nobody else puts work on it.
+//
+// Work is never put on both streams at once: while another thread's call works on
+// own a direct fence is refused, and a call that needs own waits for the direct
+// fences open in other threads.  Whoever changes the stream joins the two by an
+// event, which then covers all the work of the other one.
 class WorkStream {
  public:
+  ~WorkStream();
   operator cudaStream_t() const { return get(); }
   void set(cudaStream_t s) { own_ = s; }
   cudaStream_t own() const { return own_; }
   void hand_out() const;  // the caller gets the handle: no direct work any more
-  bool begin_direct(int device) const;  // false: not possible on this stream
+  bool begin_direct(int device) const;  // false: not possible on this stream, or not now
   bool end_direct() const;              // false: this thread is in no direct fence
 
  private:
+  friend struct CallScope;
   cudaStream_t get() const;
   cudaStream_t own_ = nullptr;
   mutable std::mutex mu_;
+  mutable std::condition_variable closed_;  // the last direct fence has ended
   mutable int device_ = -1;
+  mutable int direct_ = 0;     // threads in a direct fence
+  mutable int calls_ = 0;      // library calls in progress that work on own_
   mutable bool given_ = false;    // the handle is the caller's or was handed out
   mutable bool own_ahead_ = false;      // work on own_ the default stream has not joined
   mutable bool default_ahead_ = false;  // and the other way round
 };
+
+// Work put on `after` from here on waits for the work now on `before`.
+void order_streams(int device, cudaStream_t before, cudaStream_t after);
 
 }  // namespace spmvb
 
