@@ -872,6 +872,9 @@ int spmv_matrix_set_values(spmv_matrix A, spmv_memory memory,
       // for it (5.2 M FP64 values: 5 ms for both copies through the host).
       A->comm->require_device();
       cudaStream_t s = A->comm->stream;
+      // (Behind the legacy default stream as well, where a caller without a fence
+      // may just have computed the values.)
+      order_streams(A->comm->device, nullptr, s);
       A->h_vals_stale = true;
       for (int r = 0; r < P; ++r) {
         const int64_t nnz = A->h_rowptr[r][A->nrows[r]];
