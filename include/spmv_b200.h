@@ -221,7 +221,9 @@ int spmv_matrix_dtype(spmv_matrix A, spmv_dtype* dtype);
 int spmv_matrix_rows(spmv_matrix A, int rank, int32_t* nrows);
 int spmv_matrix_cols(spmv_matrix A, int rank, int32_t* ncols);
 int spmv_matrix_nnz(spmv_matrix A, int rank, int64_t* nnz);
-/* Matrix::mat() (Matrix.h:51-53): the host copy of rank's CSR block. */
+/* Matrix::mat() (Matrix.h:51-53): the host copy of rank's CSR block.  The arrays
+ * are the matrix's own and stay valid with it; spmv_matrix_set_values changes the
+ * values in place. */
 int spmv_matrix_csr(spmv_matrix A, int rank, const int32_t** rowptr,
                     const int32_t** colind, const void** values);
 /* Matrix::col_map()/row_map() (Matrix.h:45-48). */

@@ -827,6 +827,7 @@ int spmv_matrix_csr(spmv_matrix A, int rank, const int32_t** rowptr,
     *colind = A->h_colind[rank].data();
     fresh_host_values(A);
     *values = A->h_vals[rank].data();
+    A->h_vals_given = true;
   });
 }
 
@@ -869,7 +870,8 @@ int spmv_matrix_set_values(spmv_matrix A, spmv_memory memory,
       A->h_vals_stale = false;
     } else {
       // The device copy only: the host copy is read back when something asks
-      // for it (5.2 M FP64 values: 5 ms for both copies through the host).
+      // for it (5.2 M FP64 values: 5 ms for both copies through the host), or at
+      // once where spmv_matrix_csr has given its address to the caller.
       A->comm->require_device();
       cudaStream_t s = A->comm->stream;
       // (Behind the legacy default stream as well, where a caller without a fence
@@ -883,6 +885,7 @@ int spmv_matrix_set_values(spmv_matrix A, spmv_memory memory,
                                      values[r], nnz * es, cudaMemcpyDeviceToDevice, s));
       }
       SPMVB_CUDA(cudaStreamSynchronize(s));
+      if (A->h_vals_given) fresh_host_values(A);
     }
     // Derived copies are rebuilt on next use (the mixed solver's graph holds
     // the FP32 copy's address, so it goes too).

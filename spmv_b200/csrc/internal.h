@@ -350,6 +350,7 @@ struct spmv_matrix_s {
   std::vector<std::vector<int32_t>> h_rowptr, h_colind;
   std::vector<std::vector<unsigned char>> h_vals;
   bool h_vals_stale = false;  // the device's values are newer (fresh_host_values)
+  bool h_vals_given = false;  // the caller has their address (spmv_matrix_csr)
   std::vector<int32_t> nrows, ncols;
   // Device plans.
   spmvb::DevCsr fwd;            // A
