@@ -43,6 +43,7 @@ struct BlockWorkspace {
   // b, x, r, p, y (n x k, for the largest k solved so far), per-CTA partials,
   // state and the grid barrier's counter.
   spmvb::DevBuf b, x, r, p, y, partials, state;
+  std::vector<spmvb::DevBuf*> vectors() { return {&b, &x, &r, &p, &y}; }
 };
 
 namespace spmvb {
@@ -59,6 +60,10 @@ constexpr int LONG_ROW = 512;      // entries above which a row is the whole CTA
 // their neighbours' in L1; the solver's are one per CTA up to this size (its
 // vectors then stay in L2 between the phases).
 constexpr int SPMM_CHUNK = 4096, BCG_CHUNK = 24576;
+// Bytes of vectors a matrix keeps between block solves.  (Allocating and freeing them
+// takes 3 ms for 0.67 GB, 128^3 rows and k = 8, where 40 iterations take 15, and 5.4 ms
+// for 2.7 GB, k = 32, where they take 52.)
+constexpr size_t BCG_KEEP = size_t(1) << 30;
 
 // Right-hand sides per lane.  V consecutive ones, the vectors aligned to V
 // values (SPLIT false); or two, loaded one by one, the second missing from
@@ -642,18 +647,32 @@ void launch_spmm(spmv_matrix A, int k, const void* const* x, void* const* y,
 
 void destroy_block_workspace(BlockWorkspace* w) { delete w; }
 
-BlockWorkspace& block_workspace(spmv_matrix A, int k) {
+BlockWorkspace& block_workspace(spmv_matrix A) {
   if (!A->blk)
     A->blk = std::unique_ptr<BlockWorkspace, void (*)(BlockWorkspace*)>(new BlockWorkspace,
                                                                         destroy_block_workspace);
-  BlockWorkspace& w = *A->blk;
+  return *A->blk;
+}
+
+void reserve_block(spmv_matrix A, BlockWorkspace& w, int k) {
   w.n = A->row_map->ranges.back();
   const size_t bytes = sizeof(double) * std::max<int64_t>(w.n * k, 1);
-  for (DevBuf* v : {&w.b, &w.x, &w.r, &w.p, &w.y}) v->reserve(bytes);
+  for (DevBuf* v : w.vectors()) v->reserve(bytes);
   w.state.reserve(sizeof(BcgState));
   w.partials.reserve(sizeof(double) * 2 * MAXK * size_t(std::max(1, A->comm->num_sms)));
-  return w;
 }
+
+// At the end of a solve (also a failed one): vectors of up to BCG_KEEP bytes stay
+// with the matrix for the next one, larger ones go back to the device.
+struct BlockVectors {
+  BlockWorkspace& w;
+  ~BlockVectors() {
+    size_t bytes = 0;
+    for (DevBuf* v : w.vectors()) bytes += v->bytes;
+    if (bytes > BCG_KEEP)
+      for (DevBuf* v : w.vectors()) v->release();
+  }
+};
 
 // Block CG in the fused-halo layout over the workspace's row-major n x k
 // blocks: w.b to w.x.
@@ -778,7 +797,9 @@ int spmv_cg_block(spmv_matrix A, int nrhs, spmv_memory memory, const double* con
     cudaStream_t s = comm->stream;
     spmv_l2gmap rm = A->row_map, cm = A->col_map;
     const int P = comm->size;
-    BlockWorkspace& w = block_workspace(A, nrhs);
+    BlockWorkspace& w = block_workspace(A);
+    const BlockVectors vectors{w};
+    reserve_block(A, w, nrhs);
     const cudaMemcpyKind in = memory == SPMV_MEMORY_HOST ? cudaMemcpyHostToDevice
                                                          : cudaMemcpyDeviceToDevice;
     const cudaMemcpyKind outk = memory == SPMV_MEMORY_HOST ? cudaMemcpyDeviceToHost
