@@ -1280,8 +1280,8 @@ float time_iterations(CgWorkspace& w, cudaStream_t s, int its) {
 }
 
 // Chooses between the graph form and the fused plans that fit, by timing 32
-// iterations of each on b = 1: the on-chip form where its vectors fit, else
-// (with a staged product)
+// iterations of each on b = 1: the on-chip form where its vectors fit, and unless
+// that is well ahead (with a staged product)
 // r in shared memory with one or two CTAs per SM (when the CTAs' rows fit),
 // or r in global memory with two CTAs of 6 stages or three of 4; and the
 // merged-update form (two grid syncs per iteration) of the 2-CTA shared and
@@ -1334,30 +1334,30 @@ void choose_form(spmv_matrix A, CgWorkspace& w) {
     return;
   }
   std::vector<FusedPlan> plans;
-  {
-    FusedPlan p0, p1, p2, p3, p4, p5, p6;
-    const bool fits = onchip && plan_onchip(A, p0);
-    if (fits) plans.push_back(std::move(p0));
-    // Where the on-chip form fits, the others have not been faster (7-point
-    // 128^3: 40.0 us per iteration against 42.4 to 55.3; 96^3: 18.9 against
-    // 22.3 to 28.9; 5-point 1024^2: 15.6 against 20.3 to 24.3), so they are not
-    // timed.
-    if (staged && !fits) {
-      if (plan_fused<CgFusedOne, true>(A, sp, p1)) plans.push_back(std::move(p1));
-      if (plan_fused<CgFusedTwo, true>(A, sp, p2)) plans.push_back(std::move(p2));
-      if (plan_fused<CgFusedTwoDeep, false>(A, sp, p3)) plans.push_back(std::move(p3));
-      if (plan_fused<CgFusedThree, false>(A, sp, p4)) plans.push_back(std::move(p4));
-      if (plan_fused<CgFusedTwo, true, true>(A, sp, p5)) plans.push_back(std::move(p5));
-      if (plan_fused<CgFusedThree, false, true>(A, sp, p6)) plans.push_back(std::move(p6));
-    }
-  }
+  auto add = [&](bool fits, FusedPlan& p) {
+    if (fits) plans.push_back(std::move(p));
+  };
+  auto add_staged = [&] {
+    FusedPlan p1, p2, p3, p4, p5, p6;
+    add(plan_fused<CgFusedOne, true>(A, sp, p1), p1);
+    add(plan_fused<CgFusedTwo, true>(A, sp, p2), p2);
+    add(plan_fused<CgFusedTwoDeep, false>(A, sp, p3), p3);
+    add(plan_fused<CgFusedThree, false>(A, sp, p4), p4);
+    add(plan_fused<CgFusedTwo, true, true>(A, sp, p5), p5);
+    add(plan_fused<CgFusedThree, false, true>(A, sp, p6), p6);
+  };
+  FusedPlan chip;
+  add(onchip && plan_onchip(A, chip), chip);
+  bool more = staged && plans.empty();  // the staged plans are in the list
+  if (more) add_staged();
   if (plans.empty()) return;
   cudaStream_t s = A->comm->stream;
   const int its = 32;
   SPMVB_CUDA(cudaDeviceSynchronize());
   cg_fill<<<std::max(1, comm->num_sms) * 4, 256, 0, s>>>(w.b.as<double>(), w.n, 1.0);
   SPMVB_CUDA(cudaGetLastError());
-  float best = time_iterations(w, s, its);
+  const float graph = time_iterations(w, s, its);
+  float best = graph;
   int pick = -1;
   for (size_t i = 0; i < plans.size(); ++i) {
     use_plan(w, plans[i]);
@@ -1366,10 +1366,22 @@ void choose_form(spmv_matrix A, CgWorkspace& w) {
               (plans[i].tmem ? ":tmem" : plans[i].rs ? ":smem" : ":global") +
               (plans[i].merged ? ":m " : " ") + std::to_string(t * 1e3f / its) +
               " us per iteration");
-    if (!w.fused) continue;  // the plan's launch was refused (graph form ran)
-    if (t < best) {
+    if (w.fused && t < best) {  // (else its launch was refused and the graph form ran)
       best = t;
       pick = int(i);
+    }
+    // Where the on-chip form is well ahead of the graph form, the staged plans have not
+    // been faster, and are not timed.  us per iteration, on chip / graph / the best
+    // staged plan: 7-point 128^3 36.7 / 55.9 / 42.4, 96^3 16.7 / 35.5 / 22.3; 5-point
+    // 1024^2 14.1 / 34.2 / 20.1; a 7-point 100^3 with its rows in random order 34.7 /
+    // 55.5 / 38.5 and 11 bands of 1.2 M such rows 59.7 / 81.7 / 74.1 (0.73, the
+    // nearest).  Where most gathers leave the CTA's rows and p and x outgrow what L2
+    // serves at once, they are: in random order 5-point 1024^2 41.3 / 47.5 / 33.1, 3
+    // bands of 1.5 M rows 39.5 / 46.0 / 31.0, 5 of 1 M 39.9 / 47.8 / 32.5 (0.83), and
+    // 7-point 120^3 94.4 / 79.6 / 63.2.
+    if (staged && !more && best >= 0.75f * graph) {
+      more = true;
+      add_staged();
     }
   }
   w.fused = false;
