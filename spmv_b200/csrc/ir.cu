@@ -1155,12 +1155,23 @@ void ir_choose_form(spmv_matrix A, IrWorkspace& w) {
   // Where every CTA's window of p fits, the other forms have not been faster (us
   // per inner iteration, on chip, the best other fused plan, graph: 27-point 96^3
   // 28.1, 41.3, 51.8; 40^3 8.1, 10.7, 24.7; 7-point 64^3 8.6, 11.3, 24.8; 5-point
-  // 1024^2 14.3, 17.3, 30.5; 1400^2 22.1, 25.4, 38.6), so nothing is timed.  Where
-  // one does not (7-point 128^3: 33.0, 31.2, 44.8), every plan that fits is.
+  // 1024^2 14.3, 17.3, 30.5; 1400^2 22.1, 25.4, 38.6), so nothing is timed; unless
+  // copying the windows is a large part of the work (mesh graphs of 14 entries per row
+  // numbered at random within 4,096: 60^3 points, 3.2 M rows of p in the windows for 3.1 M
+  // entries, 14.2 and graph 33.9, but 76^3, 4.6 M for 6.2 M, 41.9 and 44.4, 92^3, 7.2 M
+  // for 11 M, 62.2 and 60.0, 100^3 75.9 and 72.4; 7-point 112^3, 5.1 M for 9.8 M, 25.5,
+  // 26.1, 38.1): then the graph form is, and the fused plans where the on-chip form is
+  // not well ahead of it (cg.cu).  Where a window does not fit (7-point 128^3:
+  // 33.0, 31.2, 44.8), every plan that fits is.
+  bool full = false;
   if (onchip && ir_use_onchip(A, w)) {
-    bool full = true;
-    for (const bat::OnchipCta& c : w.onchip.ctas) full = full && c.full;
-    if (full) return;
+    full = true;
+    int64_t rows = 0;
+    for (const bat::OnchipCta& c : w.onchip.ctas) {
+      full = full && c.full;
+      rows += c.wrows;
+    }
+    if (full && (rows <= (int64_t(4) << 20) || 2 * rows <= A->fwd.nz_total)) return;
     w.fused = w.fused_tm = false;
   }
   std::vector<FusedPlan> plans;
@@ -1183,13 +1194,15 @@ void ir_choose_form(spmv_matrix A, IrWorkspace& w) {
               " us per solve + refinement");
     return per_it + fixed / 100.f;
   };
-  float best = score("graph");
+  const float graph = score("graph");
+  float best = graph;
   int pick = -1;
   bool chip = false;
   if (onchip && ir_use_onchip(A, w)) {
     const float t = score("on chip");
     chip = w.fused_tm && t < best;
     if (chip) best = t;
+    if (chip && full && t < 0.75f * graph) plans.clear();
   }
   for (size_t i = 0; i < plans.size(); ++i) {
     ir_use_plan(w, plans[i]);

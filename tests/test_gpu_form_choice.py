@@ -51,3 +51,12 @@ def test_cg_rows_in_random_order(cuda_device):
     form, log = run("cg", "c1", 1024, 5, shuffled=True)
     assert "cg form 1:tmem:m" in log and "cg form 2:smem:m" in log
     assert form != "tmem:m"
+
+def test_mixed_with_narrow_windows(cuda_device):
+    form, log = run("mixed", "c3", 64, 9)
+    assert form == "tmem:m" and "cg_mixed form" not in log
+
+
+def test_mixed_with_wide_windows(cuda_device):
+    form, log = run("mixed", "c2", 112, 7)
+    assert "cg_mixed form graph" in log and "cg_mixed form on chip" in log
