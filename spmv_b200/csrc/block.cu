@@ -12,7 +12,7 @@
 // a chain of dependent loads (row pointer, column, X).  So each lane keeps
 // SPMM_BATCH entries in flight and issues every batch whole (a tail of single
 // entries costs one chain each), the next row's pointers are loaded a row
-// ahead, and a CTA takes chunks of neighbouring rows (RowChunks).  Rows longer
+// ahead, and a CTA takes a chunk of neighbouring rows.  Rows longer
 // than LONG_ROW entries are left to the whole CTA.  Against one right-hand
 // side per lane, batches of four and a tail (FP64, 7-point 96^3, 4 ranks):
 // k = 2 24.7 -> 20.2 us, k = 8 69.8 -> 59.3, k = 16 133 -> 104 (3.0 TB/s of
@@ -112,20 +112,6 @@ __device__ __forceinline__ void st_run(const R& r, T* p, const T (&v)[R::V]) {
   }
 }
 
-// Rows are dealt to the CTAs in chunks of consecutive rows (global numbering):
-// chunk q is [q rows, (q + 1) rows).  A chunk's neighbouring rows share X rows
-// in the CTA's L1, and chunks in flight are consecutive, so the X rows that
-// rows further apart share (the next plane of a grid) are read from DRAM
-// once.
-struct RowChunks {
-  int64_t rows, total;  // rows per chunk, rows in all
-  int count;
-  __host__ __device__ int64_t begin(int64_t q) const { return q * rows; }
-  __host__ __device__ int64_t end(int64_t q) const {
-    return (q + 1) * rows < total ? (q + 1) * rows : total;
-  }
-};
-
 // acc += the row's entries below e from j on, in batches of SPMM_BATCH
 // consecutive entries at j, j + step, ...  Every batch is issued whole: past
 // the end it repeats the last entry and the sum skips it.  (X may be written
@@ -152,93 +138,94 @@ __device__ __forceinline__ void spmm_entries(const R& r, const int32_t* cols, co
   }
 }
 
-// Rows [g0, g1) (global numbering) of Y = A X, by the whole CTA, KL lanes per
-// row: f(P, row, run, sums) once per row and lane that has right-hand sides.
+// Rows [lo, hi) of a rank's Y = A X, by the whole CTA, KL lanes per row: f(P, row, run,
+// sums) once per row and lane that has right-hand sides.
 template <typename T, int NT, int KL, class R, class F>
-__device__ __forceinline__ void spmm_rows(const SpmvArgs& a, int k, int64_t g0, int64_t g1,
-                                          F&& f) {
+__device__ __forceinline__ void spmm_rows(const PartArg& P, int k, int lo, int hi, F&& f) {
   constexpr int V = R::V;
   __shared__ T group_sums[NT * V];
   __shared__ unsigned int long_mask[NT / 32];
   const int tid = int(threadIdx.x), grp = tid / KL;
   const R run(tid % KL, k);
-  int64_t row0 = 0;
-  for (int p = 0; p < a.nparts; ++p) {
-    const PartArg& P = a.part[p];
-    const int64_t first = row0;
-    row0 += P.nrows;
-    const int lo = int(max(g0, first) - first), hi = int(min(g1, row0) - first);
-    if (g0 >= row0 || g1 <= first || lo >= hi) continue;
-    const T* xc = static_cast<const T*>(P.x) + (run.on ? run.c0 : 0);
-    const T* vals = static_cast<const T*>(P.vals);
-    int row = lo + grp;
-    int s = 0, e = 0, any_long = 0;
-    if (row < hi) {
-      s = __ldg(P.rowptr + row);
-      e = __ldg(P.rowptr + row + 1);
+  const T* xc = static_cast<const T*>(P.x) + (run.on ? run.c0 : 0);
+  const T* vals = static_cast<const T*>(P.vals);
+  int row = lo + grp;
+  int s = 0, e = 0, any_long = 0;
+  if (row < hi) {
+    s = __ldg(P.rowptr + row);
+    e = __ldg(P.rowptr + row + 1);
+  }
+  while (row < hi) {
+    const int next = row + NT / KL;
+    int sn = 0, en = 0;
+    if (next < hi) {
+      sn = __ldg(P.rowptr + next);
+      en = __ldg(P.rowptr + next + 1);
     }
-    while (row < hi) {
-      const int next = row + NT / KL;
-      int sn = 0, en = 0;
-      if (next < hi) {
-        sn = __ldg(P.rowptr + next);
-        en = __ldg(P.rowptr + next + 1);
-      }
-      if (e - s > LONG_ROW) {
-        any_long = 1;
-      } else {
+    if (e - s > LONG_ROW) {
+      any_long = 1;
+    } else {
+      T acc[V];
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[i] = T(0);
+      spmm_entries<T>(run, P.cols, vals, xc, k, s, e, SPMM_BATCH, acc);
+      if (run.on) f(P, row, run, acc);
+    }
+    row = next;
+    s = sn;
+    e = en;
+  }
+  if (!__syncthreads_or(any_long)) return;
+  // Long rows, in row order: every group takes batches in
+  // turn; the groups' sums are added in group order.
+  for (int r0 = lo; r0 < hi; r0 += NT) {
+    const int mine = r0 + tid;
+    const bool is_long =
+        mine < hi && __ldg(P.rowptr + mine + 1) - __ldg(P.rowptr + mine) > LONG_ROW;
+    const unsigned int m = __ballot_sync(0xffffffffu, is_long);
+    if ((tid & 31) == 0) long_mask[tid >> 5] = m;
+    __syncthreads();
+    for (int w = 0; w < NT / 32; ++w)
+      for (unsigned int left = long_mask[w]; left != 0; left &= left - 1) {
+        const int lrow = r0 + 32 * w + __ffs(left) - 1;
+        const int ls = __ldg(P.rowptr + lrow), le = __ldg(P.rowptr + lrow + 1);
         T acc[V];
 #pragma unroll
         for (int i = 0; i < V; ++i) acc[i] = T(0);
-        spmm_entries<T>(run, P.cols, vals, xc, k, s, e, SPMM_BATCH, acc);
-        if (run.on) f(P, row, run, acc);
-      }
-      row = next;
-      s = sn;
-      e = en;
-    }
-    if (!__syncthreads_or(any_long)) continue;
-    // Long rows, in row order: every group takes batches in
-    // turn; the groups' sums are added in group order.
-    for (int r0 = lo; r0 < hi; r0 += NT) {
-      const int mine = r0 + tid;
-      const bool is_long =
-          mine < hi && __ldg(P.rowptr + mine + 1) - __ldg(P.rowptr + mine) > LONG_ROW;
-      const unsigned int m = __ballot_sync(0xffffffffu, is_long);
-      if ((tid & 31) == 0) long_mask[tid >> 5] = m;
-      __syncthreads();
-      for (int w = 0; w < NT / 32; ++w)
-        for (unsigned int left = long_mask[w]; left != 0; left &= left - 1) {
-          const int lrow = r0 + 32 * w + __ffs(left) - 1;
-          const int ls = __ldg(P.rowptr + lrow), le = __ldg(P.rowptr + lrow + 1);
-          T acc[V];
+        spmm_entries<T>(run, P.cols, vals, xc, k, ls + grp * SPMM_BATCH, le,
+                        SPMM_BATCH * (NT / KL), acc);
 #pragma unroll
-          for (int i = 0; i < V; ++i) acc[i] = T(0);
-          spmm_entries<T>(run, P.cols, vals, xc, k, ls + grp * SPMM_BATCH, le,
-                          SPMM_BATCH * (NT / KL), acc);
+        for (int i = 0; i < V; ++i) group_sums[tid * V + i] = acc[i];
+        __syncthreads();
+        if (grp == 0 && run.on) {
 #pragma unroll
-          for (int i = 0; i < V; ++i) group_sums[tid * V + i] = acc[i];
-          __syncthreads();
-          if (grp == 0 && run.on) {
-#pragma unroll
-            for (int i = 0; i < V; ++i) {
-              T t = T(0);
-              for (int g = 0; g < NT / KL; ++g) t += group_sums[g * KL * V + run.c0 + i];
-              acc[i] = t;
-            }
-            f(P, lrow, run, acc);
+          for (int i = 0; i < V; ++i) {
+            T t = T(0);
+            for (int g = 0; g < NT / KL; ++g) t += group_sums[g * KL * V + run.c0 + i];
+            acc[i] = t;
           }
-          __syncthreads();
+          f(P, lrow, run, acc);
         }
-      __syncthreads();
-    }
+        __syncthreads();
+      }
+    __syncthreads();
   }
 }
 
+// Each CTA a chunk of `rows` rows of one rank, which it finds by bisection.  (Chunks
+// across the ranks' borders, found by passing the ranks in turn, cost small products 1 to
+// 2 us of latency: every rank is a constant line of its own, and a chunk over a border
+// takes two passes that all others wait for.  FP64, 8,000 7-point rows over 8 ranks, k = 8
+// 6.2 us, now 4.1 to 5; 884,736 rows over 4 ranks, k = 8 59.4 and 55.6, k = 32 195 and
+// 178.)
 template <typename T, int KL, class R>
 __global__ void __launch_bounds__(BBS, BCPS)
-    spmm_kernel(const __grid_constant__ SpmvArgs a, const RowChunks ch, int k) {
-  spmm_rows<T, BBS, KL, R>(a, k, ch.begin(blockIdx.x), ch.end(blockIdx.x),
+    spmm_kernel(const __grid_constant__ SpmvArgs a, int rows, int k) {
+  const PartArg& P = a.part[find_part(a, blockIdx.x)];
+  const int lo = (int(blockIdx.x) - P.block_begin) * rows;
+  const int hi = P.nrows - lo < rows ? P.nrows : lo + rows;
+  if (lo >= hi) return;
+  spmm_rows<T, BBS, KL, R>(P, k, lo, hi,
                            [&](const PartArg& P, int row, const R& run, const T(&acc)[R::V]) {
                              st_run<T>(run, static_cast<T*>(P.y) + int64_t(row) * k + run.c0,
                                        acc);
@@ -294,6 +281,31 @@ __global__ void __launch_bounds__(BBS)
 // ---------------------------------------------------------------------------
 // Block CG
 // ---------------------------------------------------------------------------
+// The rows of all ranks in equal chunks of consecutive rows (global numbering): chunk q
+// is [q rows, (q + 1) rows).
+struct RowChunks {
+  int64_t rows, total;  // rows per chunk, rows in all
+  int count;
+  __host__ __device__ int64_t begin(int64_t q) const { return q * rows; }
+  __host__ __device__ int64_t end(int64_t q) const {
+    return (q + 1) * rows < total ? (q + 1) * rows : total;
+  }
+};
+
+// g(P, lo, hi) for each rank's rows among [g0, g1) (global numbering).
+template <class G>
+__device__ __forceinline__ void each_rank(const SpmvArgs& a, int64_t g0, int64_t g1, G&& g) {
+  int64_t row0 = 0;
+  for (int p = 0; p < a.nparts; ++p) {
+    const PartArg& P = a.part[p];
+    const int64_t first = row0;
+    row0 += P.nrows;
+    const int lo = int(max(g0, first) - first), hi = int(min(g1, row0) - first);
+    if (g0 >= row0 || g1 <= first || lo >= hi) continue;
+    g(P, lo, hi);
+  }
+}
+
 struct BcgState {
   double rr0[MAXK], rr[MAXK];
   int status[MAXK], its[MAXK];
@@ -430,16 +442,17 @@ __global__ void __launch_bounds__(CBS)
 #pragma unroll
     for (int i = 0; i < R::V; ++i) py[i] = 0.0;
     for (int q = blockIdx.x; q < ch.count; q += gridDim.x)
-      spmm_rows<double, CBS, KL, R>(
-          a, k, ch.begin(q), ch.end(q),
-          [&](const PartArg& P, int row, const R& run, const double(&s)[R::V]) {
-            const int64_t o = int64_t(row) * k + run.c0;
-            double pv[R::V];
-            ld_run<double>(run, static_cast<const double*>(P.xown) + o, pv);
-            st_run<double>(run, static_cast<double*>(P.y) + o, s);
+      each_rank(a, ch.begin(q), ch.end(q), [&](const PartArg& Q, int lo, int hi) {
+        spmm_rows<double, CBS, KL, R>(
+            Q, k, lo, hi, [&](const PartArg& P, int row, const R& run, const double(&s)[R::V]) {
+              const int64_t o = int64_t(row) * k + run.c0;
+              double pv[R::V];
+              ld_run<double>(run, static_cast<const double*>(P.xown) + o, pv);
+              st_run<double>(run, static_cast<double*>(P.y) + o, s);
 #pragma unroll
-            for (int i = 0; i < R::V; ++i) py[i] += pv[i] * s[i];
-          });
+              for (int i = 0; i < R::V; ++i) py[i] += pv[i] * s[i];
+            });
+      });
     ++epoch;
     if (!column_sums<R::V>(py, KL, CBS, c, parts(), epoch * gridDim.x, sh)) break;
     if (tid < k) {
@@ -546,22 +559,24 @@ int run_width(int k, size_t es, int P, const void* const* x, const void* const* 
   return v > 1 ? v : 0;
 }
 
-// Every row in one launch table (each rank's arrays; the CTAs' rows come from
-// the cut table).
-SpmvArgs spmm_args(spmv_matrix A, const int32_t* cols, size_t es, const void* const* x,
-                   void* const* y, const void* const* xown) {
-  SpmvArgs a;
-  fill_spmv_args(a, A->fwd, cols, es, x, y, xown, BBS, 1);
-  return a;
+// Rows per chunk: at most `most`, so that the chunks are whole rounds of `grid` CTAs, of
+// which `lost` may go to ranks that do not end with a whole chunk.
+int64_t chunk_rows(int64_t total, int grid, int64_t most, int lost) {
+  const int64_t rounds = std::max<int64_t>(1, (total + grid * most - 1) / (grid * most));
+  const int64_t slots = std::max<int64_t>(1, grid * rounds - lost);
+  return std::max<int64_t>(1, (total + slots - 1) / slots);
+}
+int64_t total_rows(spmv_matrix A) {
+  int64_t total = 0;
+  for (const DevPart& D : A->fwd.parts) total += D.nrows;
+  return total;
 }
 
-// Chunks of at most `most` rows, in whole rounds of `grid` CTAs (equal
-// shares).
+// Block CG's chunks.
 RowChunks row_chunks(spmv_matrix A, int grid, int64_t most) {
   RowChunks ch{};
-  for (const DevPart& D : A->fwd.parts) ch.total += D.nrows;
-  const int64_t rounds = std::max<int64_t>(1, (ch.total + grid * most - 1) / (grid * most));
-  ch.rows = std::max<int64_t>(1, (ch.total + grid * rounds - 1) / (grid * rounds));
+  ch.total = total_rows(A);
+  ch.rows = chunk_rows(ch.total, grid, most, 0);
   ch.count = int((ch.total + ch.rows - 1) / ch.rows);
   return ch;
 }
@@ -626,7 +641,6 @@ void launch_spmm(spmv_matrix A, int k, const void* const* x, void* const* y,
                                 dim3(t.nblocks), dim3(BBS), args, 0, stream));
     return;
   }
-  const SpmvArgs a = spmm_args(A, A->fwd.cols.as<int32_t>(), es, x, y, nullptr);
   const int kl = lanes_for(k, v ? v : 2);
   const void* fn;
   if (k == 1)
@@ -638,11 +652,15 @@ void launch_spmm(spmv_matrix A, int k, const void* const* x, void* const* y,
     fn = v == 4   ? spmm_fn<float, Run<4, false>>(kl)
          : v == 2 ? spmm_fn<float, Run<2, false>>(kl)
                   : spmm_fn<float, Run<2, true>>(kl);
-  RowChunks ch = row_chunks(A, std::max(1, A->comm->num_sms) * BCPS,
-                            std::max(128, SPMM_CHUNK / k));
-  if (ch.count == 0) return;
-  void* args[] = {const_cast<SpmvArgs*>(&a), &ch, &k};
-  SPMVB_CUDA(cudaLaunchKernel(fn, dim3(ch.count), dim3(BBS), args, 0, stream));
+  // Chunks in flight are consecutive, so the X rows that rows further apart share (the
+  // next plane of a grid) are read from DRAM once.
+  int rows = int(chunk_rows(total_rows(A), std::max(1, A->comm->num_sms) * BCPS,
+                            std::max(128, SPMM_CHUNK / k), A->comm->size - 1));
+  SpmvArgs a;
+  fill_spmv_args(a, A->fwd, A->fwd.cols.as<int32_t>(), es, x, y, nullptr, rows, INT32_MAX);
+  if (a.nblocks == 0) return;
+  void* args[] = {&a, &rows, &k};
+  SPMVB_CUDA(cudaLaunchKernel(fn, dim3(a.nblocks), dim3(BBS), args, 0, stream));
 }
 
 void destroy_block_workspace(BlockWorkspace* w) { delete w; }
@@ -689,8 +707,9 @@ void block_cg(spmv_matrix A, BlockWorkspace& w, int k, int max_its, double rtol,
     own[q] = w.p.as<double>() + off;
     ys[q] = w.y.as<double>() + off;
   }
-  SpmvArgs a = spmm_args(A, A->fwd.cols_global.as<int32_t>(), sizeof(double), xs.data(),
-                         ys.data(), own.data());
+  SpmvArgs a;
+  fill_spmv_args(a, A->fwd, A->fwd.cols_global.as<int32_t>(), sizeof(double), xs.data(), ys.data(),
+                 own.data(), BBS, 1);
   BcgPtrs c{};
   c.b = w.b.as<double>();
   c.x = w.x.as<double>();
