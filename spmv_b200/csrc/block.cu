@@ -234,12 +234,9 @@ __global__ void __launch_bounds__(BBS, BCPS)
 
 // One right-hand side per lane, KL lanes per row, CTAs striding over tiles of
 // BBS / KL rows; batches of four entries and a tail of single ones, in 32
-// registers (every warp slot of the SM taken).  For an odd number of
-// right-hand sides (or vectors off a 16-byte boundary) on rows of several
-// batches, where twice the warps are worth more than two right-hand sides
-// per lane loaded one by one (FP64, 60^3 rows: k = 7, 27-point 51 us against
-// 58, mesh 34 against 43; k = 31, 148 against 172 and 91 against 102; rows of
-// 7 entries, 96^3: k = 7, 70 against 66, k = 31, 255 against 219).
+// registers (every warp slot of the SM taken).  For products whose lanes cannot
+// load aligned runs of X, and whose rows either take several batches of
+// spmm_kernel or leave most of one empty (use_walk).
 template <typename T, int KL>
 __global__ void __launch_bounds__(BBS)
     spmm_walk_kernel(const __grid_constant__ SpmvArgs a, int k) {
@@ -596,6 +593,7 @@ const void* spmm_fn(int kl) {
 template <typename T>
 const void* spmm_walk_fn(int kl) {
   switch (kl) {
+    case 1: return (const void*)spmm_walk_kernel<T, 1>;
     case 2: return (const void*)spmm_walk_kernel<T, 2>;
     case 4: return (const void*)spmm_walk_kernel<T, 4>;
     case 8: return (const void*)spmm_walk_kernel<T, 8>;
@@ -619,6 +617,34 @@ const void* bcg_fn(int kl) {
 
 }  // namespace
 
+// Whether a product with run width v (run_width) is spmm_walk_kernel's; us by it and by
+// spmm_kernel:
+//  * rows of several batches, single loads (odd k or unaligned vectors): twice the warps
+//    are worth more than two right-hand sides per lane loaded one by one (FP64, 60^3 rows:
+//    k = 7, 27-point 51 and 58, mesh 34 and 43; k = 31, 148 and 172, 91 and 102; rows of 7
+//    entries, 96^3: k = 7, 70 and 66, k = 31, 255 and 219);
+//  * rows of at most 4 entries, of which a batch of 8 repeats half (FP64, rows of 3: 600,000
+//    k = 3 14.4 and 20.2, 2 M k = 3 58.8 and 64.2; FP32 600,000 k = 7 24.5 and 25.7, 2 M k
+//    = 7 98.3 and 95.4, k = 17 358 and 304); in FP64 also the wide even k that leave lanes
+//    over while X and Y stay in L2 (150,000 k = 24 24.6 and 29.0, 600,000 125 and 115);
+//  * rows of at most 6 in FP64 while X and Y are well inside L2 (5-point 420^2 k = 7 12.3
+//    and 14.4, 520^2 k = 3 10.3 and 12.3, 800^2 k = 5, 51 MB, 40.4 and 37.1);
+//  * one right-hand side, a thread per row: rows of at most 6 entries (FP64 600,000 of 3
+//    6.5 and 8.2, 1200^2 5-point 22.6 and 24.0, but 7-point 96^3 14.4 and 14.4, 40^3 5.2
+//    and 4.1; FP32 2 M of 3 12.3 and 18.5), in FP32 of at most 8 where there are many
+//    (7-point 88^3 8.8 and 9.3, 108^3 14.4 and 15.9, but 72^3 7.8 and 6.2).
+static bool use_walk(const DevCsr& C, int64_t rows, int k, int v, size_t es, int l2_bytes) {
+  if (C.max_row > LONG_ROW) return false;  // some row is for a whole CTA
+  const bool f64 = es == 8;
+  if (v == 0 && C.mean_row > SPMM_BATCH) return true;
+  if (C.max_row > 4 * SPMM_BATCH) return false;
+  const int64_t bytes = 2 * rows * k * int64_t(es);  // of X and Y
+  if (k == 1) return C.mean_row <= (f64 || 32 * bytes <= l2_bytes ? 6.0 : 8.0);
+  if (v != 0) return f64 && C.mean_row <= 4.0 && k > 8 && 2 * bytes <= l2_bytes;
+  if (C.mean_row <= 4.0) return f64 || k < 16;
+  return f64 && C.mean_row <= 6.0 && 4 * bytes <= l2_bytes;
+}
+
 // y[r] (nrows x k) = A[r] x[r] (ncols x k) for all ranks, device pointers.
 void launch_spmm(spmv_matrix A, int k, const void* const* x, void* const* y,
                  cudaStream_t stream) {
@@ -628,9 +654,7 @@ void launch_spmm(spmv_matrix A, int k, const void* const* x, void* const* y,
   const size_t es = dtype_size(A->dtype);
   const int v = run_width(k, es, A->comm->size, x, y);
   const bool f64 = A->dtype == SPMV_FLOAT64;
-  // Right-hand sides that cannot be loaded in aligned runs, on rows that take
-  // several batches: the tile walk, unless some row is for a whole CTA.
-  if (v == 0 && A->fwd.mean_row > SPMM_BATCH && A->fwd.max_row <= LONG_ROW) {
+  if (use_walk(A->fwd, total_rows(A), k, v, es, A->comm->l2_bytes)) {
     const int kl = lanes_for(k, 1);
     SpmvArgs t;
     fill_spmv_args(t, A->fwd, A->fwd.cols.as<int32_t>(), es, x, y, nullptr, BBS / kl,
