@@ -336,12 +336,10 @@ __global__ void __launch_bounds__(NW * 32, 1) onchip_groups(const __grid_constan
         tmem_ld(t, rv);
         tmem_st(t + C, y);
         tmem_wait_ld(rv);
-        if (row) {
-          const double yd = double(y);
-          in[0] += double(ps[at]) * yd;
-          in[1] += double(rv.get()) * yd;
-          in[2] += yd * yd;
-        }
+        const double yd = double(y);  // (a lane without a row: r and y are 0, p is not its own)
+        in[0] += double(row ? ps[at] : T(0)) * yd;
+        in[1] += double(rv.get()) * yd;
+        in[2] += yd * yd;
       };
       if (!(me.full
                 ? oc_pass<true, MX, T, CI, U, D>(view(), ring, ps, w0, rows, pg, row_sums)
@@ -359,41 +357,45 @@ __global__ void __launch_bounds__(NW * 32, 1) onchip_groups(const __grid_constan
       // C, two slices in flight per warp.
       const T alpha = T(sv.alpha), beta = T(sv.beta);
       const int n = me.nitems;
+      auto update = [&](auto count, int j, uint32_t t) {
+        constexpr int B = decltype(count)::value;
+        int4 h[B];
+        int l[B];
+        T pv[B];
+        Tm r[B], y[B], d[B];
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+          h[b] = items[j + b * NW];
+          l[b] = h[b].y - w0 + lane;
+          pv[b] = ps[l[b]];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+          tmem_ld(t + b * CS, r[b]);
+          tmem_ld(t + b * CS + C, y[b]);
+          tmem_ld(t + b * CS + 2 * C, d[b]);
+        }
+        tmem_wait_ld(r, y, d);
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+          const T rn = r[b].get() - alpha * y[b].get(), pn = rn + beta * pv[b];
+          __syncwarp();
+          tmem_st(t + b * CS, rn);
+          tmem_st(t + b * CS + 2 * C, d[b].get() + alpha * pv[b]);
+          if (exists(h[b])) {
+            ps[l[b]] = pn;
+            if (me.size > 1) __stcg(pg + w0 + l[b], pn);
+          }
+          rr += double(rn) * double(rn);
+        }
+      };
       uint32_t t = tm;
       for (int j = warp; j < n; j += 2 * NW, t += 2 * CS) {
-        const bool two = j + NW < n;
-        const int4 h0 = items[j], h1 = items[two ? j + NW : j];
-        const int l0 = h0.y - w0 + lane, l1 = h1.y - w0 + lane;
-        const T p0 = ps[l0], p1 = ps[l1];
-        Tm r0, y0, d0, r1, y1, d1;
-        __syncwarp();
-        tmem_ld(t, r0);
-        tmem_ld(t + C, y0);
-        tmem_ld(t + 2 * C, d0);
-        const uint32_t t1 = two ? t + CS : t;  // (the first's again: not used)
-        tmem_ld(t1, r1);
-        tmem_ld(t1 + C, y1);
-        tmem_ld(t1 + 2 * C, d1);
-        tmem_wait_ld(r0, y0, d0, r1, y1, d1);
-        const T rn0 = r0.get() - alpha * y0.get(), pn0 = rn0 + beta * p0;
-        tmem_st(t, rn0);
-        tmem_st(t + 2 * C, d0.get() + alpha * p0);
-        if (exists(h0)) {
-          ps[l0] = pn0;
-          if (me.size > 1) __stcg(pg + w0 + l0, pn0);
-        }
-        rr += double(rn0) * double(rn0);
-        if (two) {
-          const T rn1 = r1.get() - alpha * y1.get(), pn1 = rn1 + beta * p1;
-          __syncwarp();
-          tmem_st(t + CS, rn1);
-          tmem_st(t + CS + 2 * C, d1.get() + alpha * p1);
-          if (exists(h1)) {
-            ps[l1] = pn1;
-            if (me.size > 1) __stcg(pg + w0 + l1, pn1);
-          }
-          rr += double(rn1) * double(rn1);
-        }
+        if (j + NW < n)
+          update(std::integral_constant<int, 2>{}, j, t);
+        else
+          update(std::integral_constant<int, 1>{}, j, t);
       }
       __syncwarp();
       tmem_wait_st();
