@@ -1306,7 +1306,8 @@ void choose_form(spmv_matrix A, CgWorkspace& w) {
                       (!A->kernel_set || A->kernel == SPMV_KERNEL_STAGED);
   // The other fused kernels stream the staged product's tile table.
   const bool staged = sp.kind == ProductKind::Staged && cg_tiles(A, sp).ok;
-  if (!onchip && !staged) return;
+  // (A staged plan asked for on a matrix with another product: the graph form.)
+  if (mode.empty() || mode == "1:tmem:m" ? !onchip && !staged : !staged) return;
   if (staged) {
     const DevCsr::StagedTable& tiles = cg_tiles(A, sp);
     w.tiles = tiles.desc.as<StagedDesc>();
@@ -1319,7 +1320,6 @@ void choose_form(spmv_matrix A, CgWorkspace& w) {
     FusedPlan p;
     bool fits = false;
     if (mode == "1:tmem:m") fits = onchip && plan_onchip(A, p);
-    else if (!staged) fits = false;
     else if (mode == "1:smem") fits = plan_fused<CgFusedOne, true>(A, sp, p);
     else if (mode == "2:smem") fits = plan_fused<CgFusedTwo, true>(A, sp, p);
     else if (mode == "1:global") fits = plan_fused<CgFusedOne, false>(A, sp, p);

@@ -1132,7 +1132,8 @@ void ir_choose_form(spmv_matrix A, IrWorkspace& w) {
   SPMVB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, comm->device));
   if (!coop) return;
   const bool tiles = staged && ir_tiles(A, w.p32, true).ok;
-  if (!onchip && !tiles) return;
+  // (A staged plan asked for on a matrix with another product: the graph form.)
+  if (mode.empty() || mode == "1:tmem:m" ? !onchip && !tiles : !tiles) return;
   w.bar.reserve(sizeof(unsigned long long));
   if (tiles) {
     ir_args(A, w, w.p32, true, w.fa32);
@@ -1143,8 +1144,7 @@ void ir_choose_form(spmv_matrix A, IrWorkspace& w) {
     FusedPlan p;
     bool fits = false;
     if (mode == "1:tmem:m" && onchip && ir_use_onchip(A, w)) return;
-    if (!tiles) fits = false;
-    else if (mode == "2:smem") fits = ir_plan<IrFusedTwo, true>(A, w, p);
+    if (mode == "2:smem") fits = ir_plan<IrFusedTwo, true>(A, w, p);
     else if (mode == "2:global") fits = ir_plan<IrFusedTwo, false>(A, w, p);
     else if (mode == "3:global") fits = ir_plan<IrFusedThree, false>(A, w, p);
     require(fits, "spmv: SPMV_B200_CG_MIXED_FUSED must be 0 or a fused plan that fits this "
