@@ -75,8 +75,10 @@ struct OcScalars {
 };
 
 // The decisions after the sum of A (one thread; every CTA of the group makes
-// the same ones from the same totals).  T: the precision alpha is applied in.
-template <typename T>
+// the same ones from the same totals).  T: the precision alpha is applied in; MX: an
+// iteration that breaks down counts (as in the mixed solve's other forms; not in the
+// batch's).
+template <typename T, bool MX>
 __device__ __forceinline__ void oc_step(OcScalars& v, const double (&tot)[4], int kmax,
                                         double rtol2, double delta2) {
   const double rr = tot[3];
@@ -91,6 +93,7 @@ __device__ __forceinline__ void oc_step(OcScalars& v, const double (&tot)[4], in
   if (py == 0.0 || !isfinite(py)) {
     v.status = SPMV_ERROR_BREAKDOWN;
     v.go = 0;
+    if (MX) v.its += 1;
     return;
   }
   const double al = double(T(rr / py));
@@ -348,7 +351,7 @@ __global__ void __launch_bounds__(NW * 32, 1) onchip_groups(const __grid_constan
       __syncwarp();
       tmem_wait_st();
       if (!(ok = group_sum(in, tot))) break;
-      if (tid == 0) oc_step<T>(sv, tot, a.kmax, a.rtol2, a.delta2);
+      if (tid == 0) oc_step<T, MX>(sv, tot, a.kmax, a.rtol2, a.delta2);
       named_sync(1, NT);
     }
     if (!sv.go) break;

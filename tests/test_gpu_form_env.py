@@ -34,3 +34,14 @@ def test_staged_plan_on_a_matrix_without_a_staged_product(monkeypatch, cuda_devi
         assert M.cg_form(solver) == ("graph", 0, None)
         rel = np.linalg.norm(b - A.scipy() @ x[0][:n]) / np.linalg.norm(b)
         assert rel < 1.5e-10
+
+
+@pytest.mark.parametrize("plan", ["0", "2:smem", "1:tmem:m"])
+def test_mixed_breakdown_counts_its_iteration(monkeypatch, cuda_device, plan):
+    monkeypatch.setenv("SPMV_B200_CG_MIXED_FUSED", plan)
+    W = gen.workload("c2", 24)
+    Z = gen.CSR(W.A.rowptr, W.A.cols, 0.0 * W.A.vals, W.A.ncols)
+    comm, cm, rm, M, D = build(Z, 1)
+    M.set_kernel("staged", 7)
+    with pytest.raises(S.SpmvError, match="breakdown .* after 1 iterations"):
+        S.cg_mixed(comm, M, [W.b.copy()], 100, 1e-8)
