@@ -949,10 +949,12 @@ std::vector<OnchipKernel> onchip_kernels(spmv_matrix A) {
   const bool d = A->fwd.d16;
   const int64_t w = A->fwd.max_row;
   // Rows of at most 5 entries: pairs of slices (an item of one is mostly
-  // overhead: 1024^2 5-point, 20.0 us per iteration against 15.6).  At 7
-  // entries pairs gain nothing (128^3: 40.0 us against 42.7).  Wider rows: four
-  // columns a copy (rows of 13 to 25 entries, 216k rows: 15.8 us against 18.2
-  // with eight).
+  // overhead: 5-point 1024^2 17.6 us per iteration against 14.2, 512^2 8.8 against
+  // 8.0).  At 7 entries pairs gain little (96^3 17.1 and 17.1, 64^3 9.2 against 9.5)
+  // and do not fit 128^3.  Wider rows: four columns a copy, the values read early
+  // (with eight early, rows of 13 to 25 entries, 216k rows, 18.2 us against 15.8; eight
+  // read late are level there, 15.3 and 15.6, and 24.1 and 24.9 at 439k rows, and ahead
+  // on 27-point rows, 64^3 18.4 and 20.9, 96^3 42.0 and 50.8).
   if (w <= 5) return {onchip_kernel<20, 5, 2, 2, true>(d), onchip_kernel<16, 5, 2, 2, false>(d)};
   if (w <= 7) return {onchip_kernel<24, 7, 2, 1, true>(d), onchip_kernel<20, 7, 2, 1, false>(d)};
   return {onchip_kernel<24, 4, 3, 1, false>(d), onchip_kernel<16, 4, 3, 1, false>(d)};

@@ -1154,8 +1154,8 @@ void ir_choose_form(spmv_matrix A, IrWorkspace& w) {
   }
   // Where every CTA's window of p fits, the other forms have not been faster (us
   // per inner iteration, on chip, the best other fused plan, graph: 27-point 96^3
-  // 28.1, 41.3, 51.8; 40^3 8.1, 10.7, 24.7; 7-point 64^3 8.6, 11.3, 24.8; 5-point
-  // 1024^2 14.3, 17.3, 30.5; 1400^2 22.1, 25.4, 38.6), so nothing is timed; unless
+  // 28.6, 41.3, 51.8; 40^3 8.2, 10.7, 24.7; 7-point 64^3 8.6, 11.3, 24.8; 5-point
+  // 1024^2 14.7, 17.3, 30.5; 1400^2 22.1, 25.4, 38.6), so nothing is timed; unless
   // copying the windows is a large part of the work (mesh graphs of 14 entries per row
   // numbered at random within 4,096: 60^3 points, 3.2 M rows of p in the windows for 3.1 M
   // entries, 14.2 and graph 33.9, but 76^3, 4.6 M for 6.2 M, 41.9 and 44.4, 92^3, 7.2 M

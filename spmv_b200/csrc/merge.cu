@@ -37,8 +37,15 @@ namespace {
 constexpr int MBS = 256;  // threads per CTA
 constexpr int IPT = 8;    // merge items per thread
 constexpr int TILE = MBS * IPT;
-constexpr int SHORT = 32;  // entries of a tile that one thread sums
-constexpr int MID = 256;   // and one warp
+// Entries of a tile that one thread sums, and one warp.  A thread per row is the
+// fastest where the rows' lengths are odd multiples of few banks (4 M entries, us per
+// product: rows of 17, 18.5 with SHORT = 32 and 39.0 with 16; of 33, 28.7 and with 64
+// 18.5; but of 32, 31.2 and with 16 28.7, of 64, 22.6 and with 64 32.7: the lanes of
+// equal rows then share banks).  MID = 128: rows of 200 31.5 against 18.5; MID = 512: of
+// 300 17.8 against 26.6, of 600 20.8 against 22.4; 300,007 power-law rows 34.6, between
+// 33.8 and 36.5 with any of these.
+constexpr int SHORT = 32;
+constexpr int MID = 256;
 
 // Smallest row count i in [lo, hi] (rows consumed) of the split point on
 // diagonal d: the first i with rowend(i) > d - i - 1, rowend(i) = rowptr[i + 1].

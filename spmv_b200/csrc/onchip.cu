@@ -38,8 +38,8 @@
 // and 5 columns: 63 us in the lockstep kernel, 5.6 here; 24 of 22,000 and 32
 // columns, the chip full, 105 and 24.
 // One matrix, mixed (the fused form of ir.cu before): 27-point 96^3 41.3 us per
-// iteration, now 28.1 (its entries are 22 at the rate of a copy); 5-point 1024^2
-// 17.3 and 14.3, 200 x 180 19.1 and 5.8 (as a CUDA graph before); 27-point 40^3
+// iteration, now 28.6 (its entries are 22 at the rate of a copy); 5-point 1024^2
+// 17.3 and 14.7, 200 x 180 19.1 and 5.8 (as a CUDA graph before); 27-point 40^3
 // 10.7 and 8.1.
 #include <algorithm>
 #include <cmath>
